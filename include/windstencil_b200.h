@@ -128,13 +128,13 @@ typedef struct ws_metrics {
 } ws_metrics;
 
 /* Kernel selection.  All zeros (the default) and tile_x < 0 select the line
- * passes: three barrier-free passes (x, y, z) in which each lane marches one
- * grid line (with tile_x < 0, threads = 32 x warps per CTA, or 0 for the
- * tuned count).  Any other tile_x, tile_y, threads select the fused tile
- * sweep: a CTA of `threads` threads owns tile_x x tile_y columns and sweeps
- * them along z; scan_z caps the planes of one sweep (0: no cap, each
- * persistent CTA sweeps its whole share of planes).  Both give the same
- * results, CLOSURE faces included. */
+ * passes: three passes (x, y, z) in which each lane marches one grid line
+ * (with tile_x < 0, threads = 0, or 256 in FP64 and 512 mixed).  Any other
+ * tile_x, tile_y, threads select the fused tile sweep: a CTA of `threads`
+ * threads owns tile_x x tile_y columns and sweeps them along z; scan_z caps
+ * the planes of one sweep (0: no cap, each persistent CTA sweeps its whole
+ * share of planes; < 0: the line passes instead).  Both give the same results
+ * to rounding, CLOSURE faces included. */
 typedef struct ws_tile {
     int32_t tile_x, tile_y, scan_z, threads;
 } ws_tile;
@@ -481,7 +481,9 @@ WS_API int  ws_batch_rhs(ws_batch* b, ws_stream_t stream);
 WS_API int  ws_batch_step(ws_batch* b, int nsteps, ws_stream_t stream);
 /* per-grid status (0, WS_ERR_NONFINITE or WS_ERR_TIMEOUT); synchronises `stream` */
 WS_API int  ws_batch_status(ws_batch* b, int* status, ws_stream_t stream);
-/* times the compiled tile shapes on this batch's RHS and keeps the fastest */
+/* times the line passes and the compiled tile shapes on this batch's RHS and
+ * keeps the fastest; *chosen is its tile selection (scan_z = -1: the line
+ * passes) */
 WS_API int  ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream);
 
 /* ------------------------------------------------------------------------ */

@@ -243,14 +243,23 @@ int tile_index(const ws_grid* g, ws_tile tile, bool stage, int* cfg) {
 // Fill RhsArgs and launch; shared by the drop-in entry and the solver.
 bool use_pencil(const ws_grid* g, ws_tile tile) {
     (void)g;
-    if (tile.tile_x < 0) return true;
+    if (tile.tile_x < 0 || tile.scan_z < 0) return true;
     return !(tile.tile_x || tile.tile_y || tile.threads);
 }
 
 namespace {
+// tile_x < 0 may name the warps per CTA that a line pass has always run with
+// (8 in FP64, 16 mixed) or leave them open
 int check_pencil(const ws_grid* g, ws_tile tile) {
-    (void)g;
+    if (tile.tile_x >= 0) {
+        int cfg = 0;
+        return tile_index(g, tile, false, &cfg);
+    }
     if (tile.threads % 32) return fail(WS_ERR_INVALID, "line passes: threads = 32 x warps");
+    const int warps = g->precision == WS_MIXED ? 16 : 8;
+    if (tile.threads > 0 && tile.threads / 32 != warps)
+        return fail(WS_ERR_UNSUPPORTED, "line passes: " + std::to_string(warps) +
+                                            " warps per CTA");
     return WS_OK;
 }
 }  // namespace
@@ -261,8 +270,7 @@ int rhs_enqueue(const ws_grid* g, ws_job job, const ws_field prims[5], const ws_
         int rc = check_pencil(g, tile);
         if (rc) return rc;
         const RhsArgs a = make_rhs_args(g, job, prims, m, du, 0, 1);
-        return launch_rhs_pencil(a, g->precision, g->metrics_uniform != 0, tile.threads / 32, 0,
-                                 false, st);
+        return launch_rhs_pencil(a, g->precision, g->metrics_uniform != 0, 0, false, st);
     }
     int cfg = 0;
     int rc = tile_index(g, tile, false, &cfg);
@@ -289,8 +297,7 @@ int rhs_stage_enqueue(const ws_grid* g, const ws_field p_in[6], ws_soa f_in, ws_
         const ws_field p5[5] = {p_in[0], p_in[1], p_in[2], p_in[3], p_in[5]};
         RhsArgs a = make_rhs_args(g, job, p5, nullptr, du, 0, 1);
         if ((rc = set_rhs_stage(a, g, f_in, fn, f_out, p_out, dt, status))) return rc;
-        return launch_rhs_pencil(a, g->precision, true, tile.threads / 32, krk,
-                                 dvis.ptr != nullptr, st);
+        return launch_rhs_pencil(a, g->precision, true, krk, dvis.ptr != nullptr, st);
     }
     int cfg = 0;
     int rc = tile_index(g, tile, true, &cfg);

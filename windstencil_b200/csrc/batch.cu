@@ -181,7 +181,7 @@ int batch_kernel_cfg(const std::vector<GridState*>& grids, ws_tile tile) {
     if (tile.tile_x < 0) return -1;
     if (tile.tile_x || tile.tile_y || tile.threads) {
         const int c = find_tile_cfg(tile.tile_x, tile.tile_y, tile.threads);
-        return c < 0 ? -2 : c;
+        return c < 0 ? -2 : tile.scan_z < 0 ? -1 : c;
     }
     return -1;
 }
@@ -240,15 +240,15 @@ int BatchRunner::build(const std::vector<GridState*>& grids, int cfg, int zc, cu
     }
     const size_t o_gt = o;
     o = align256(o_gt + n_gtab * sizeof(int2));
-    const size_t o_woff = o;           // line passes: 3 x (n + 1) work prefixes
-    const size_t bytes = align256(o_woff + 3 * (size_t)(n + 1) * sizeof(long));
+    const size_t o_woff = o;           // line passes: kWorkTables x (n + 1) work prefixes
+    const size_t bytes = align256(o_woff + kWorkTables * (size_t)(n + 1) * sizeof(long));
     host_.assign(bytes, 0);
     unsigned char* h = host_.data();
     if (!items.empty())
         std::memcpy(h + o_items, items.data(), items.size() * sizeof(int4));
     int2* hgt = reinterpret_cast<int2*>(h + o_gt);
     long* hw = reinterpret_cast<long*>(h + o_woff);
-    for (int dir = 0; dir < 3; ++dir) {
+    for (int dir = 0; dir < kWorkTables; ++dir) {
         long* w = hw + dir * (n + 1);
         w[0] = 0;
         for (int i = 0; i < n; ++i) w[i + 1] = w[i] + pencil_pass_work(grids[i]->g, dir);
@@ -570,8 +570,9 @@ int ws_batch_status(ws_batch* b, int* status, ws_stream_t stream) {
 // Times the candidate kernels on the first RK stage of this batch (ghost
 // fill + RHS and stage update; the current state is left as it was) and
 // keeps the fastest; returns its tile selection in *chosen.  Candidates: the
-// line passes (tile_x = -1) and every compiled tile shape of the fused
-// kernel with two sweep caps.
+// line passes (the default tile shape with scan_z = -1, which any set_tile
+// takes as the line passes) and every compiled tile shape of the fused kernel
+// with two sweep caps.
 int ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream) {
     if (!b) return fail(WS_ERR_INVALID, "batch is NULL");
     cudaStream_t st = (cudaStream_t)stream;
@@ -580,7 +581,8 @@ int ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream) {
     WS_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     ws_tile best_tile{0, 0, 0, 0};
-    std::vector<ws_tile> cand{ws_tile{-1, 0, 0, 0}};
+    const TileCfg dc = tile_cfg(default_cfg(b->states[0].g.precision, true));
+    std::vector<ws_tile> cand{ws_tile{dc.bx, dc.by, -1, dc.threads}};
     for (int c = 0; c < num_tile_cfgs(); ++c)
         for (int cap : {0, 32}) {
             const TileCfg tc = tile_cfg(c);

@@ -202,44 +202,41 @@ __device__ __forceinline__ double face_flux<float, false>(const float* bp, int p
 // value otherwise.  In y the ring kernel drops the M term of the last cell;
 // the face above it (f == n, used by that cell only) carries M of face n-1
 // instead of its own, which cancels the M term in that cell's difference.
-// The same from the two stencils as arrays: sp[k] = F+ and sm[k] = F- of
-// cell f-4+k.
-__device__ __forceinline__ double closure_value_arr(const double sp[8], const double sm[8], int f,
-                                                    int n, bool lo, bool hi, bool ydir) {
-    double P, M, num, den;
-    if (lo && f == 0) P = sp[4];
-    else if (lo && f == 1) P = w5::p_lift(sp + 1);
-    else if (lo && f == 2) P = w5::p_lift_plus(sp + 1);
-    else if ((lo && f == 3) || (hi && f == n - 2)) P = w5::p3(sp + 1);
-    else if (hi && f == n - 1) P = w5::p_right_plus(sp + 1);
-    else if (hi && f == n)
-        P = ydir ? sp[3] + 0.5 * w5::minmod2(sp[3] - sp[2], sp[3] - sp[2])
-                 : 1.5 * sp[3] - 0.5 * sp[2];
-    else {
-        double t[8];
+// The two terms from the stencils as arrays: sp[k] = F+ and sm[k] = F- of cell
+// f-4+k.
+__device__ __forceinline__ double closure_p_arr(const double sp[8], int f, int n, bool lo,
+                                                bool hi, bool ydir) {
+    if (lo && f == 0) return sp[4];
+    if (lo && f == 1) return w5::p_lift(sp + 1);
+    if (lo && f == 2) return w5::p_lift_plus(sp + 1);
+    if ((lo && f == 3) || (hi && f == n - 2)) return w5::p3(sp + 1);
+    if (hi && f == n - 1) return w5::p_right_plus(sp + 1);
+    if (hi && f == n)
+        return ydir ? sp[3] + 0.5 * w5::minmod2(sp[3] - sp[2], sp[3] - sp[2])
+                    : 1.5 * sp[3] - 0.5 * sp[2];
+    double t[8], num, den;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] = sp[k];
-        weno7_symbo_nd<false>(t, num, den);
-        P = sp[3] + num / den;
-    }
-    if (lo && f == 0) M = w5::m_lift(sm + 2);
-    else if (lo && f == 1) M = w5::m_lift_plus(sm + 2);
-    else if ((lo && (f == 2 || f == 3)) || (hi && f == n - 3)) M = w5::m3(sm + 2);
-    else if (hi && f == n - 2) M = w5::m_right_plus(sm + 2);
-    else if (hi && f == n - 1)
-        M = ydir ? sm[4] - 0.5 * w5::minmod2(sm[4] - sm[3], sm[4] - sm[3])
-                 : 0.5 * sm[4] + 0.5 * sm[3];
-    else if (hi && f == n)      // y: M of face n-1 (see above)
-        M = ydir ? sm[3] - 0.5 * w5::minmod2(sm[3] - sm[2], sm[3] - sm[2])
-                 : 0.5 * sm[3] + 0.5 * sm[2];
-    else {
-        double t[8];
+    for (int k = 0; k < 8; ++k) t[k] = sp[k];
+    weno7_symbo_nd<false>(t, num, den);
+    return sp[3] + num / den;
+}
+__device__ __forceinline__ double closure_m_arr(const double sm[8], int f, int n, bool lo,
+                                                bool hi, bool ydir) {
+    if (lo && f == 0) return w5::m_lift(sm + 2);
+    if (lo && f == 1) return w5::m_lift_plus(sm + 2);
+    if ((lo && (f == 2 || f == 3)) || (hi && f == n - 3)) return w5::m3(sm + 2);
+    if (hi && f == n - 2) return w5::m_right_plus(sm + 2);
+    if (hi && f == n - 1)
+        return ydir ? sm[4] - 0.5 * w5::minmod2(sm[4] - sm[3], sm[4] - sm[3])
+                    : 0.5 * sm[4] + 0.5 * sm[3];
+    if (hi && f == n)      // y: M of face n-1 (see above)
+        return ydir ? sm[3] - 0.5 * w5::minmod2(sm[3] - sm[2], sm[3] - sm[2])
+                    : 0.5 * sm[3] + 0.5 * sm[2];
+    double t[8], num, den;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) t[k] = sm[7 - k];
-        weno7_symbo_nd<false>(t, num, den);
-        M = sm[4] + num / den;
-    }
-    return P + M;
+    for (int k = 0; k < 8; ++k) t[k] = sm[7 - k];
+    weno7_symbo_nd<false>(t, num, den);
+    return sm[4] + num / den;
 }
 
 template <typename CT>
@@ -251,7 +248,7 @@ __device__ __forceinline__ double closure_value(const CT* prow, const CT* mrow, 
         sp[k] = (double)prow[k * stride];
         sm[k] = (double)mrow[k * stride];
     }
-    return closure_value_arr(sp, sm, f, n, lo, hi, ydir);
+    return closure_p_arr(sp, f, n, lo, hi, ydir) + closure_m_arr(sm, f, n, lo, hi, ydir);
 }
 
 // face f of a direction with n cells needs a closure value

@@ -1,498 +1,604 @@
-// pencil_impl.cuh -- BF3W inviscid RHS as three barrier-free line passes.
+// pencil_impl.cuh -- BF3W inviscid RHS as three line passes.
 //
 // Replaces, like the fused kernel (bf3w_rhs_impl.cuh), the reference's
 // split_Jac3d_Stager_Warming_ker (src/kernels/OCFD_split.cpp:36-3918) and
-// its boundary-ring kernel (src/solver/OCFD_NS_Jacobian3d.cpp:828-2530), with
-// the same per-point arithmetic (ws_device.cuh).  The fused kernel sweeps a
-// 2D column footprint along z with CTA barriers between its split and face
-// intervals and recomputes the footprint's halo splits and edge faces.  Here
-// every lane owns one grid line along the pass direction and marches it
-// alone: per point it computes the Steger-Warming split of the point four
-// ahead into a private 8-slot ring in shared memory, reconstructs the face
-// above the current point from the ring (WENO7-SYMBO P and M), and adds the
-// face difference of the point to du.  No lane reads another lane's ring, so
-// there is no barrier and no halo work across lines; a warp's lanes own 32
-// consecutive lines of the flattened pair of the other two axes, so there
-// are no partial tiles, and each warp takes an equal contiguous share of the
-// (line group, position) space.  The primitives of the next split and the
-// du of the next point are loaded a step ahead, so that their latency
-// overlaps the current step's reconstructions.
+// its boundary-ring kernel (src/solver/OCFD_NS_Jacobian3d.cpp:828-2530).  The
+// fused kernel sweeps a 2D column footprint along z and recomputes the
+// footprint's halo splits and edge faces; here a RHS is three passes, x (du =,
+// or += onto viscous terms already stored in du), y (+=) and z (+=, or in
+// stage mode the SSP-RK3 stage update and the primitives of the new state),
+// and every pass marches whole grid lines, so no split and no face is
+// computed twice (except an 8-point prologue per line segment).
 //
-// A RHS is three passes, x (du =, or += onto viscous terms already stored in
-// du), y (+=) and z (+=, or in stage mode the SSP-RK3 stage update and the
-// primitives of the new state, as the fused kernel's epilogue).  du goes
-// through HBM between the passes, which the compute-bound passes absorb
-// (~320 B/cell against ~7.3 kFLOP/cell).
+// Ten warps (two such thread groups to a CTA, one CTA per SM) take a group of
+// lines (32; 64 in the mixed form, two per lane in packed FP32x2): lane =
+// line, warp = one sign of the split flux of one conserved variable.  Every lane takes its split flux through the
+// streaming reconstruction of line_weno.cuh, whose state -- differences and
+// waiting indicators, 22 values -- stays in its registers.  After marching a
+// chunk of five points, the five F+ warps split the chunk after next (one
+// point each, all ten components, into a ring in shared memory) and the five
+// F- warps write the previous chunk out (one point each, all five variables);
+// a component's ring entry is read by its own lane only, which leaves the
+// cell's result in its place.  Operands of both arrive by cp.async issued a
+// chunk ahead into per-thread slots.  A warp enters its exchange when all
+// have finished theirs of the chunk before (a barrier split into arrival and
+// wait), so no warp waits for another unless it is a whole march ahead.
+//
+// Why this split: with all five variables in one lane (the earlier form) the
+// reconstruction could keep nothing between faces, so each face took 190 FP64
+// operations from a ring of splits that also held the SM to 8 warps.  One
+// sign of one variable fits 96 registers: 20 warps per SM and 118 operations
+// per face.  Both signs in a lane would take 112, but their state spilled (10
+// warps at 168 registers: y pass 1.14 ms at 600x128x128, 15 warps at 128: 1.36
+// ms).  Measured at 600x128x128, earlier form -> this one: FP64 x .980 -> .543,
+// y .808 -> .580, z .818 -> .581, z with the stage .948 -> .632 ms; mixed x .487
+// -> .335, y .363 -> .328, z .373 -> .304 ms.  FP64 pipe 65-68% active (ncu);
+// an FMA with three distinct registers takes it 3 cycles instead of 2, and
+// fixed-latency waits and the exchange take the rest.  du goes through HBM
+// between the passes (~320 B/cell).
 #pragma once
+#include <algorithm>
 #include <type_traits>
 
 #include "bf3w_rhs_impl.cuh"
+#include "line_weno.cuh"
+#include "pencil_lane.cuh"
 
 namespace ws {
 
-template <typename CT>
-struct PencilLayout {
-    static constexpr int RS = 10 * 32;            // ring slot stride (CT), lanes inner
-    static constexpr int WARP = 8 * RS;           // one warp's ring
-};
-
 enum PencilMode { P_STORE = 0, P_ADD = 1, P_STAGE = 2 };
 
-// Face value of variable v of face f (direction of n cells, CLOSURE flags lo /
-// hi, ydir: the y forms) from a lane's ring column `col` of ns slots (slot
-// stride 10 x 32, the stencil from slot s0 on): the closure value next to a
-// CLOSURE face, the WENO7 value elsewhere.  Not inlined: the steps near the
-// line ends call it, and one copy keeps the march loops' code within the
-// instruction cache (inlined into those steps, the closure code doubled the
-// y pass's time through instruction fetch stalls).
-template <typename CT>
-__device__ __noinline__ double pencil_closure_face(const CT* col, int s0, int ns, int v, int f,
-                                                   int n, int lo, int hi, bool ydir) {
-    constexpr int RS = 10 * 32;
-    if (closure_face(f, n, lo, hi)) {
-        double sp[8], sm[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int sk = s0 + k < ns ? s0 + k : s0 + k - ns;
-            const CT* e = col + sk * RS;
-            sp[k] = (double)e[v * 32];
-            sm[k] = (double)e[(5 + v) * 32];
-        }
-        return closure_value_arr(sp, sm, f, n, lo, hi, ydir);
+// C points per chunk (the march is unrolled C times, more than the longest
+// lag, so the lagged values rotate through registers).  Ring of four chunks --
+// being written out, marched, ready, being split -- the 8-point prologue in
+// the last 8 slots.  A cell's result goes to the slot of the point just taken
+// (OFF = 0), or with CLOSURE faces, which read 7 points of history, 8 slots
+// further back (two more chunks keep it from the splits).
+template <typename V, bool CLO>
+struct PencilLayout {
+    static constexpr int NL = LineVal<V>::NL, GL = 32 * NL;
+    static constexpr int C = 5, NT = 320, HT = NT / 2;   // threads of a group, of one role
+    static constexpr int SLOTS = (CLO ? 6 : 4) * C, OFF = CLO ? 8 : 0;
+    static_assert(SLOTS >= 4 * C + OFF && SLOTS >= 2 * C + 8, "ring");
+    // slot stride padded for the x pass, whose lanes write (and read back)
+    // neighbouring slots at once; unpadded these would share their banks
+    static constexpr int RS = 10 * 32 + 3;               // V per slot
+    static constexpr size_t RING = ((size_t)SLOTS * RS * sizeof(V) + 15) / 16 * 16;
+    // operands brought ahead, per line of a role thread: 5 primitives (F+
+    // warps); du, and in stage mode fn and f (F- warps)
+    template <int MODE>
+    static constexpr size_t bytes() {                    // of one group
+        return RING +
+               (size_t)(5 + (MODE == 0 ? 0 : MODE == 1 ? 5 : 15)) * NL * HT * sizeof(double) +
+               GL * 2 * sizeof(int) + 16;                // the group's lines, two mbarriers
     }
-    return face_flux<CT, true>(col + s0 * RS + v * 32, 5 * 32, RS, ns - s0, ns * RS);
+    static_assert(sizeof(V) == 8, "one 8-byte value per lane and component");
+};
+
+// 12 x (closure value - central value) of component c (0..4 F+, 5..9 F-) at
+// face f (direction of n cells, CLOSURE flags lo / hi, ydir: the y forms) for
+// line half h, from the lane's ring column's stencil of 8 points starting at
+// slot s0 of `slots`.  Not inlined: only the steps near CLOSURE ends call it,
+// and one copy keeps the march within the instruction cache.
+template <typename V>
+__device__ __noinline__ double pencil_closure_face(const V* col, int s0, int slots, int rs,
+                                                   bool minus, int h, int f, int n, int lo,
+                                                   int hi, bool ydir) {
+    using CT = typename LineVal<V>::CT;
+    double s[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int sk = s0 + k < slots ? s0 + k : s0 + k - slots;
+        s[k] = (double)reinterpret_cast<const CT*>(col + sk * rs)[h];
+    }
+    const double val = minus ? closure_m_arr(s, f, n, lo, hi, ydir)
+                             : closure_p_arr(s, f, n, lo, hi, ydir);
+    return 12.0 * val - (7.0 * (s[3] + s[4]) - (s[2] + s[5]));
 }
 
-// March length, first LAP position and line count of pass DIR over the job
-// of `a`; the pass's work is its line groups (32 lines) x positions.
-template <int DIR>
+// Barrier of thread group tg of a CTA.
+__device__ __forceinline__ void pencil_sync(int tg) {
+    __syncwarp();
+    asm volatile("barrier.cta.sync %0, 320;" ::"r"(tg + 1) : "memory");
+}
+// A group's phases: its ten warps arrive at the two mbarriers in turn.
+__device__ __forceinline__ void pencil_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void pencil_init_bars(unsigned char* first, size_t stride) {
+    for (int g = 0; g < 2; ++g)
+        for (int b = 0; b < 2; ++b)
+            mbar_init(reinterpret_cast<uint64_t*>(first + g * stride) + b, 10);
+}
+
+// March length and work of pass DIR over the job of `a`: line groups of GL
+// lines x positions.
+template <int DIR, int GL>
 __device__ __forceinline__ long pencil_work(const RhsArgs& a, int& L) {
     const int nxj = a.ex - a.sx, nyj = a.ey - a.sy, nzj = a.ez - a.sz;
     L = DIR == 0 ? nxj : (DIR == 1 ? nyj : nzj);
     const long NL = DIR == 0 ? (long)nyj * nzj : (DIR == 1 ? (long)nxj * nzj : (long)nxj * nyj);
-    return (NL + 31) / 32 * L;
+    return (NL + GL - 1) / GL * L;
 }
 
-// One segment of pass DIR (0 x, 1 y, 2 z): positions p0 .. p0+len-1 of the
-// lines of group grp of the job of `a`, this lane's line marched with the
-// lane's ring column `ring`.  CLO (y pass): faces next to a CLOSURE face of
-// the grid (a.clo) take the closure rules of closure_value_arr; the lanes of
-// a warp sit at the same y, so the branch is uniform.
-template <int DIR, typename CT, bool UNI, int MODE, bool CLO = false>
-__device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, CT* ring, long grp,
-                                               int p0, int len) {
-    static_assert(MODE != P_STAGE || (DIR == 2 && UNI), "stage update: z pass, Cartesian");
-    static_assert(!CLO || DIR == 1, "closure faces: y pass (the x pass is pencil_x_segment)");
+// Positions p0 .. p0+len-1 of the lines of a group of a grid of the pass;
+// ahead: the place in that grid where the next piece starts (-1: none).
+struct PencilPiece {
+    int grid, p0, len;
+    long grp, ahead;
+};
+
+// One piece of pass DIR (0 x, 1 y, 2 z) over the job of `a`, by thread group
+// tg of a CTA.  CLO: faces next to a
+// CLOSURE face of the direction take the closure rules (the lines of a group
+// march the same position, so the test is uniform).
+template <int DIR, typename V, bool UNI, int MODE, bool CLO>
+__device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsigned char* smem,
+                                               int tg, unsigned& phase,
+                                               const PencilPiece& piece) {
+    const long grp = piece.grp;
+    const int p0 = piece.p0, len = piece.len;
+    static_assert(MODE != P_STAGE || (DIR == 2 && UNI && LineVal<V>::NL == 1),
+                  "stage update: z pass, Cartesian, FP64");
+    static_assert(!CLO || DIR != 2, "closure faces: x and y passes");
+    using P = PencilLayout<V, CLO>;
+    using CT = typename LineVal<V>::CT;
+    constexpr int C = P::C, NL = P::NL, RS = P::RS, HT = P::HT;
     constexpr bool ADD = MODE != P_STORE;
-    using P = PencilLayout<CT>;
-    const int lane = threadIdx.x & 31;
-    const SplitK<CT> k = {CT(a.eps2), CT(a.hrg), CT(a.c1), CT(a.c3), CT(a.gm1)};
+    const int gt = threadIdx.x - tg * P::NT, lane = gt & 31, warp = gt >> 5;
+    const bool minus = warp >= 5;
+    V* ring = reinterpret_cast<V*>(smem);
     const int nxj = a.ex - a.sx, nyj = a.ey - a.sy, nzj = a.ez - a.sz;
     const int n1 = DIR == 0 ? nyj : nxj;              // fastest line axis
-    const long NL = (long)n1 * (DIR == 2 ? nyj : nzj);
-    const int m0 = DIR == 0 ? a.sx : (DIR == 1 ? a.sy : a.sz);
-    const int mlast = (DIR == 0 ? a.nx : (DIR == 1 ? a.ny : a.nz)) + 7;   // last LAP index
-    const double rh = DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz);
+    const int nlines = n1 * (DIR == 2 ? nyj : nzj);
+    const int ms = (DIR == 0 ? a.sx : (DIR == 1 ? a.sy : a.sz)) + p0;
     const size_t vs = (size_t)a.du_pitch * a.du_ly * a.du_lz;            // du variable stride
-    const size_t fvs = MODE == P_STAGE ? (size_t)a.fn.pitch * a.fn.length_Y * a.fn.length_Z : 0;
-    long l = grp * 32 + lane;
-    const bool valid = l < NL;
-    if (!valid) l = NL - 1;
-    const int c1 = (int)(l % n1), c2 = (int)(l / n1);
-    // LAP coordinates of march position m on this lane's line
-    auto X = [&](int m) { return DIR == 0 ? m : a.sx + c1; };
-    auto Y = [&](int m) { return DIR == 1 ? m : (DIR == 0 ? a.sy + c1 : a.sy + c2); };
-    auto Z = [&](int m) { return DIR == 2 ? m : a.sz + c2; };
-    auto load = [&](int m, double q[5]) {
-        const int x = X(m), y = Y(m), z = Z(m);
-#pragma unroll
-        for (int f = 0; f < 5; ++f) q[f] = ldg_prim(a, f, x, y, z);
+    const int line0 = (int)grp * P::GL;
+
+    // ---- exchange: this thread's point sx of each chunk on line sln (and sln +
+    // 32); its operand slots, [operand][half][thread]
+    const int rt = minus ? gt - HT : gt;
+    const int sx = DIR == 0 ? rt % C : rt >> 5;
+    const int sln = DIR == 0 ? rt / C : lane;
+    double* slot = reinterpret_cast<double*>(smem + P::RING);
+    auto prim_slot = [&](int f, int h) { return slot + (f * NL + h) * HT + rt; };
+    auto cell_slot = [&](int f, int h) {
+        return slot + 5 * NL * HT + (f * NL + h) * HT + rt;
     };
-    auto split_into = [&](int m, const double q[5]) {
-        const int x = X(m), y = Y(m), z = Z(m);
-        CT out[10];
-        split_point<DIR, UNI, CT>(a, k, q[0], q[1], q[2], q[3], q[4], x, y, z, out);
-        CT* dst = ring + (m & 7) * P::RS;
+    // a point on each of the thread's lines: position m, the lines' two fixed
+    // coordinates (from a table of the group's lines, so that neither they
+    // nor addresses made of them are kept over the march)
+    struct Pt {
+        int m, c1[NL], c2[NL];
+        __device__ __forceinline__ int x(int h) const { return DIR == 0 ? m : c1[h]; }
+        __device__ __forceinline__ int y(int h) const {
+            return DIR == 1 ? m : (DIR == 0 ? c1[h] : c2[h]);
+        }
+        __device__ __forceinline__ int z(int h) const { return DIR == 2 ? m : c2[h]; }
+    };
+    int2* lines = reinterpret_cast<int2*>(smem + P::template bytes<MODE>() - 16 - P::GL * sizeof(int2));
+    auto point = [&](int m, int ln) {
+        Pt p;
+        p.m = m;
+#pragma unroll
+        for (int h = 0; h < NL; ++h) {
+            const volatile int* c = &lines[ln + 32 * h].x;
+            p.c1[h] = c[0];
+            p.c2[h] = c[1];
+        }
+        return p;
+    };
+
+    // ---- splits
+    auto prim_at = [&](int f, const Pt& p, int h) {
+        return a.prim[f] + lap_index(p.x(h), p.y(h), p.z(h), a.ppitch[f], a.ny);
+    };
+    auto pack = [&](const double (&e)[NL]) -> V {
+        if constexpr (NL == 1) return e[0];
+        else return make_float2((float)e[0], (float)e[1]);
+    };
+    auto split_into = [&](const V (&q)[5], const Pt& p, int s, int ln) {
+        const LineSplitK<V> k = {vset<V>(a.eps2), vset<V>(0.5 * a.hrg), vset<V>(a.c1),
+                                 vset<V>(0.5 + a.c3)};
+        V g[3], out[10];
+        if (!UNI) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double e[NL];
+#pragma unroll
+                for (int h = 0; h < NL; ++h)
+                    e[h] = ldg_met(a, 3 * DIR + c, p.x(h), p.y(h), p.z(h));
+                g[c] = pack(e);
+            }
+        }
+        line_split<DIR, UNI, V>(q[0], q[1], q[2], q[3], q[4], g[0], g[1], g[2], k, out);
+        V* dst = ring + s * RS + ln;
 #pragma unroll
         for (int c = 0; c < 10; ++c) dst[c * 32] = out[c];
     };
-    // du offset of march position m (job-relative); in stage mode the
-    // conserved state has du's shape, offset by the interior origin
-    auto du_at = [&](int m) {
-        return (size_t)(X(m) - a.sx) +
-               (size_t)a.du_pitch * ((size_t)(Y(m) - a.sy) + (size_t)a.du_ly * (size_t)(Z(m) - a.sz));
-    };
-    auto f_at = [&](int m) { return soa_index(a.fn, X(m) - 4, Y(m) - 4, Z(m) - 4, 0); };
-    // face value of variable v above march position m (ring stencil from
-    // slot s0 = (m - 3) & 7; face index m - 3 of the direction); the
-    // closure test is compiled only into the steps of the closure zones
-    const bool clo = CLO && (a.clo[2] | a.clo[3]);
-    auto face = [&](int s0, int m, int v, auto cl) -> double {
-        if constexpr (decltype(cl)::value)
-            return pencil_closure_face<CT>(ring, s0, 8, v, m - 3, a.ny, a.clo[2], a.clo[3], true);
-        else
-            return face_flux<CT, true>(ring + s0 * P::RS + v * 32, 5 * 32, P::RS, 8 - s0,
-                                       8 * P::RS);
-    };
-
-    const int ms = m0 + p0;
-    for (int m = ms - 4; m < ms + 4; ++m) {
-        double q[5];
-        load(m, q);
-        split_into(m, q);
-    }
-    double qn[5], dn[5], fnn[5], fin[5];
-    load(ms + 4, qn);
-    auto load_cell = [&](int m) {      // du (and the stage operands) of point m
-        if (ADD) {
-            const size_t o = du_at(m);
+    // this thread's point of chunk k: primitives fetched ahead, then split into
+    // the ring at slot `base` of the chunk
+    auto fetch_prims = [&](int k) {
+        const int i = k * C + sx;
+        if (i < len) {
+            const Pt p = point(ms + 4 + i, sln);
 #pragma unroll
-            for (int v = 0; v < 5; ++v) dn[v] = a.du[o + v * vs];
+            for (int f = 0; f < 5; ++f)
+#pragma unroll
+                for (int h = 0; h < NL; ++h) cp_async8(prim_slot(f, h), prim_at(f, p, h));
         }
-        if (MODE == P_STAGE) {
-            const size_t o = f_at(m);
-#pragma unroll
-            for (int v = 0; v < 5; ++v) {
-                fnn[v] = __ldg(a.fn.ptr + o + v * fvs);
-                fin[v] = krk == 1 ? 0.0 : a.f_in.ptr[o + v * fvs];
-            }
-        }
+        cp_async_commit();
     };
-    if (valid) load_cell(ms);
-    double fprev[5];
-    {
-        const int s0 = (ms - 4) & 7;
-#pragma unroll
-        for (int v = 0; v < 5; ++v)
-            fprev[v] = face(s0, ms - 1, v, std::integral_constant<bool, CLO>{});
-    }
-    auto step = [&](int m, auto cl) {
-        double q[5], dc[5], fnc[5], fic[5];
+    auto split_fetched = [&](int k, int base) {
+        const int i = k * C + sx;
+        cp_async_wait<0>();
+        if (i >= len) return;
+        Pt p;
+        if (!UNI) p = point(ms + 4 + i, sln);
+        V q[5];
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
-            q[f] = qn[f];
-            dc[f] = dn[f];
-            fnc[f] = fnn[f];
-            fic[f] = fin[f];
-        }
-        load(min(m + 5, mlast), qn);
-        if (valid && m + 1 < ms + len) load_cell(m + 1);
-        split_into(m + 4, q);
-        const int s0 = (m - 3) & 7;
-        const double J = UNI ? 1.0 : ldg_met(a, 9, X(m), Y(m), Z(m));
-        double r[5];
+            double e[NL];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) {
-            const double fc = face(s0, m, v, cl);
-            r[v] = -J * ((fc - fprev[v]) * rh);
-            fprev[v] = fc;
+            for (int h = 0; h < NL; ++h) e[h] = *prim_slot(f, h);
+            q[f] = pack(e);
         }
-        if (!valid) return;
-        if (MODE == P_STAGE) {
-            const size_t o = f_at(m);
-            double qs[5];
+        split_into(q, p, base + sx, sln);
+    };
+
+    // ---- results
+    auto du_at = [&](const Pt& p, int h) {
+        return (size_t)(p.x(h) - a.sx) +
+               (size_t)a.du_pitch * ((size_t)(p.y(h) - a.sy) +
+                                     (size_t)a.du_ly * (size_t)(p.z(h) - a.sz));
+    };
+    const size_t fvs = MODE == P_STAGE ? (size_t)a.fn.pitch * a.fn.length_Y * a.fn.length_Z : 0;
+    auto f_at = [&](const Pt& p, int h) {
+        return soa_index(a.fn, p.x(h) - 4, p.y(h) - 4, p.z(h) - 4, 0);
+    };
+    // du (and in stage mode the state) of this thread's point of chunk k, ahead
+    // of its result
+    auto fetch_cells = [&](int k) {
+        const int i = k * C + sx;
+        if (ADD && i < len) {
+            const Pt p = point(ms + i, sln);
 #pragma unroll
-            for (int v = 0; v < 5; ++v) {
-                qs[v] = ws_rk_stage(krk, fnc[v], fic[v], dc[v] + r[v], a.dt);
-                a.f_out.ptr[o + v * fvs] = qs[v];
+            for (int h = 0; h < NL; ++h) {
+                const size_t o = du_at(p, h);
+#pragma unroll
+                for (int w = 0; w < 5; ++w) cp_async8(cell_slot(w, h), a.du + o + w * vs);
+                if constexpr (MODE == P_STAGE) {
+                    const size_t fo = f_at(p, h);
+#pragma unroll
+                    for (int w = 0; w < 5; ++w)
+                        cp_async8(cell_slot(5 + w, h), a.fn.ptr + fo + w * fvs);
+                    if (krk != 1)
+#pragma unroll
+                        for (int w = 0; w < 5; ++w)
+                            cp_async8(cell_slot(10 + w, h), a.f_in.ptr + fo + w * fvs);
+                }
             }
-            store_prims(a, qs, X(m), Y(m), Z(m));
-        } else {
-            const size_t o = du_at(m);
+        }
+        if (ADD) cp_async_commit();
+    };
+    const double rh12 = (DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz)) * (1.0 / 12.0);
+    // result of this thread's point of chunk k at slot `base`
+    auto write_cells = [&](int k, int base) {
+        const int i = k * C + sx;
+        if (ADD) cp_async_wait<0>();
+        if (i >= len) return;
+        const Pt p = point(ms + i, sln);
+        int s = base + sx - P::OFF;
+        if (P::OFF > 0 && s < 0) s += P::SLOTS;
 #pragma unroll
-            for (int v = 0; v < 5; ++v) a.du[o + v * vs] = ADD ? dc[v] + r[v] : r[v];
+        for (int h = 0; h < NL; ++h) {
+            if (line0 + sln + 32 * h >= nlines) continue;
+            const double J = UNI ? 1.0 : ldg_met(a, 9, p.x(h), p.y(h), p.z(h));
+            const size_t o = du_at(p, h);
+            double r[5];
+#pragma unroll
+            for (int w = 0; w < 5; ++w) {
+                const V* e = ring + s * RS + w * 32 + sln;
+                const double sum = (double)reinterpret_cast<const CT*>(e)[h] +
+                                   (double)reinterpret_cast<const CT*>(e + 160)[h];
+                r[w] = ADD ? fma(-J * rh12, sum, *cell_slot(w, h)) : (-J * rh12) * sum;
+            }
+            if constexpr (MODE == P_STAGE) {
+                const size_t fo = f_at(p, h);
+                double qs[5];
+#pragma unroll
+                for (int w = 0; w < 5; ++w)
+                    qs[w] = ws_rk_stage(krk, *cell_slot(5 + w, h),
+                                        krk == 1 ? 0.0 : *cell_slot(10 + w, h), r[w], a.dt);
+#pragma unroll
+                for (int w = 0; w < 5; ++w) a.f_out.ptr[fo + w * fvs] = qs[w];
+                store_prims(a, qs, p.x(h), p.y(h), p.z(h));
+            } else {
+#pragma unroll
+                for (int w = 0; w < 5; ++w) a.du[o + w * vs] = r[w];
+            }
         }
     };
-    // closure zones: faces m - 3 <= 3 next to the low face, m - 3 >= n - 3
-    // next to the high face (LAP positions m <= 6 and m >= n)
-    const int me = ms + len;
-    int z1 = ms, z2 = me;
-    if (clo) {
-        z1 = a.clo[2] ? max(ms, min(7, me)) : ms;
-        z2 = a.clo[3] ? max(z1, min(a.ny, me)) : me;
+
+    // ---- faces: this warp's component on the lane's lines
+    V* col = ring + warp * 32 + lane;
+    WenoLine<V> st{};
+    V G[4]{}, qold{};              // first differences of lags 5..2; last face's value
+    const int nlo = CLO ? a.clo[DIR == 0 ? 0 : 2] : 0, nhi = CLO ? a.clo[DIR == 0 ? 1 : 3] : 0;
+    const int ncl = DIR == 0 ? a.nx : a.ny;
+    // takes ring slot s (LAP position m + 4); returns 12 x (the face above m
+    // less its central value) and in cen 12 x the central difference of cell m
+    auto push = [&](auto mi, int s, int m, V& cen) -> V {
+        constexpr bool MI = decltype(mi)::value;
+        cen = vfms(lkc<V, lk::SEVEN>(), vadd(G[1], G[2]), vadd(G[0], G[3]));
+        G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
+        V num, den;
+        weno_push<MI>(st, col[s * RS], num, den);
+        if constexpr (CLO) {
+            const int f = m - 3;
+            if (closure_face(f, ncl, nlo, nhi)) {
+                const int s0 = s >= 7 ? s - 7 : s - 7 + P::SLOTS;
+                double q[NL];
+#pragma unroll
+                for (int h = 0; h < NL; ++h)
+                    q[h] = pencil_closure_face<V>(col, s0, P::SLOTS, RS, MI, h, f, ncl, nlo, nhi,
+                                                  DIR == 1);
+                return pack(q);
+            }
+        }
+        return weno_quot(num, den);
+    };
+    auto step = [&](auto mi, int s, int m) {
+        V cen;
+        const V q = push(mi, s, m, cen);
+        const int so = P::OFF == 0 ? s : (s >= P::OFF ? s - P::OFF : s - P::OFF + P::SLOTS);
+        col[so * RS] = vadd(cen, vsub(q, qold));
+        qold = q;
+    };
+    // the march of one sign: state from the prologue's points, then chunk by
+    // chunk with the exchange after each
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P::template bytes<MODE>() - 16);
+    auto arrive = [&]() {              // end of phase `phase`
+        __syncwarp();
+        if (lane == 0) pencil_arrive(bars + (phase & 1));
+        __syncwarp();                  // no lane polls for a phase its own warp has yet to end
+        ++phase;
+    };
+    auto await_last = [&]() {          // all warps ended the phase before this one
+        const unsigned p = phase - 1;
+        if (!mbar_wait_bounded(bars + (p & 1), (p >> 1) & 1)) report_stage_timeout(a);
+    };
+    auto run = [&](auto mi) {
+        constexpr bool MI = decltype(mi)::value;
+        if (!MI) fetch_prims(2);
+        else fetch_cells(0);
+        // the first seven points only fill the state (nothing of their faces
+        // is used, so it is not computed); the eighth gives the first face
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            V num, den;
+            G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
+            weno_push<MI>(st, col[(P::SLOTS - 8 + i) * RS], num, den);
+        }
+        V cen;
+        qold = push(mi, P::SLOTS - 1, ms - 1, cen);
+        arrive();
+        // the last chunk runs in full: its steps past the segment take what the
+        // ring happens to hold and leave results that nobody writes out (a
+        // tail of single steps would cost the march its registers)
+        const int nch = (len + C - 1) / C;
+        int base = 0, bprev = P::SLOTS - C;        // slots of this chunk and the one before
+#pragma unroll 1
+        for (int k = 0; k < nch; ++k) {
+#pragma unroll
+            for (int i = 0; i < C; ++i) step(mi, base + i, ms + k * C + i);
+            await_last();
+            if (!MI) {
+                const int s = base + 2 * C;
+                split_fetched(k + 2, s < P::SLOTS ? s : s - P::SLOTS);
+                fetch_prims(k + 3);
+            } else if (k > 0) {
+                write_cells(k - 1, bprev);
+                fetch_cells(k);
+            }
+            arrive();
+            bprev = base;
+            base = base + C < P::SLOTS ? base + C : 0;
+        }
+        if (MI) {
+            await_last();
+            write_cells(nch - 1, bprev);
+        }
+    };
+
+    // ---- prologue: the table of lines, points ms-4 .. ms+3 into the last 8
+    // slots and the first two chunks
+    auto fixed = [&](int l, int& c1, int& c2) {       // a line's two fixed coordinates
+        l = min(l, nlines - 1);
+        c2 = l / n1;
+        c1 = l - c2 * n1 + (DIR == 0 ? a.sy : a.sx);
+        c2 += DIR == 2 ? a.sy : a.sz;
+    };
+    // calls f(point, index of the point, line) for this thread's points of the
+    // prologue of the piece of group g from position pp on
+    constexpr int NP = 8 + 2 * C;
+    auto prologue = [&](long g, int pp, int plen, auto f) {
+#pragma unroll 1
+        for (int t = gt; t < NP * 32; t += P::NT) {
+            const int i = DIR == 0 ? t % NP : t >> 5, ln = DIR == 0 ? t / NP : lane;
+            if (i >= plen + 8) continue;
+            Pt p;
+            p.m = ms - p0 + pp - 4 + i;
+#pragma unroll
+            for (int h = 0; h < NL; ++h)
+                fixed((int)g * P::GL + ln + 32 * h, p.c1[h], p.c2[h]);
+            f(p, i, ln);
+        }
+    };
+    prologue(grp, p0, len, [&](const Pt& p, int i, int ln) {
+        V q[5];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+            double e[NL];
+#pragma unroll
+            for (int h = 0; h < NL; ++h) e[h] = __ldg(prim_at(f, p, h));
+            q[f] = pack(e);
+        }
+        split_into(q, p, i < 8 ? P::SLOTS - 8 + i : i - 8, ln);
+        if (i == 0)
+#pragma unroll
+            for (int h = 0; h < NL; ++h) lines[ln + 32 * h] = make_int2(p.c1[h], p.c2[h]);
+    });
+    // the next piece's prologue, by whichever group takes it, waits for these
+    const long ahead = piece.ahead;
+    if (ahead >= 0) {
+        const int L = DIR == 0 ? nxj : (DIR == 1 ? nyj : nzj);
+        const long g = ahead / L;
+        prologue(g, (int)(ahead - g * L), 2 * C, [&](const Pt& p, int, int) {
+            if (p.m >= ms - p0 - 4 && p.m < ms - p0 + L + 4)
+#pragma unroll
+                for (int f = 0; f < 5; ++f)
+#pragma unroll
+                    for (int h = 0; h < NL; ++h) prefetch_l2(prim_at(f, p, h));
+        });
     }
-    int m = ms;
-    if constexpr (CLO)
-        for (; m < z1; ++m) step(m, std::true_type{});
-    for (; m < z2; ++m) step(m, std::false_type{});
-    if constexpr (CLO)
-        for (; m < me; ++m) step(m, std::true_type{});
+    pencil_sync(tg);
+    if (!minus) run(std::false_type{});
+    else run(std::true_type{});
 }
 
-// One pass along DIR over the job of `a`: every warp takes an equal
-// contiguous share of the (line group, position) space.
-template <int DIR, int WPB, typename CT, bool UNI, int MODE, bool CLO = false>
-__global__ void __launch_bounds__(WPB * 32, 1)
+// Work of one CTA: the contiguous share [pos, end) of the (line group,
+// position) space, which its two thread groups take piece by piece (a pair of
+// independent CTAs per SM ended up to 30% apart: the older one's warps are
+// served first).  A piece stays within a line group and within about a third
+// of what is left, so that the groups end together, but is not so short that
+// its 8-point prologue dominates.
+struct PencilShare {
+    unsigned long long pos;
+    long long end;
+    int minlen;
+    PencilPiece piece[2];          // of each thread group
+};
+__device__ __forceinline__ int pencil_piece(const PencilShare& s, long long pos, int line_left) {
+    const long long rem = s.end - pos;
+    const long long want = max(rem > 256 ? rem / 3 : (rem + 1) / 2, (long long)s.minlen);
+    int len = (int)min(min((want + 4) / 5 * 5, rem), (long long)line_left);   // whole chunks
+    if (line_left - len < 10) len = (int)min((long long)line_left, rem);
+    return len;
+}
+__device__ __forceinline__ void pencil_share(PencilShare& s, long total) {
+    s.pos = total * (long)blockIdx.x / (long)gridDim.x;
+    s.end = total * ((long)blockIdx.x + 1) / (long)gridDim.x;
+    s.minlen = (int)min(16LL, (s.end - (long long)s.pos + 1) / 2);
+}
+// The next piece of the share: grid_of(pos, local, total, L) gives the grid of
+// a position, the place within it, its number of places and the march length
+// of its lines.
+template <typename F>
+__device__ __forceinline__ PencilPiece pencil_take(PencilShare& s, F grid_of) {
+    long long pos = (long long)*reinterpret_cast<volatile unsigned long long*>(&s.pos);
+    while (pos < s.end) {
+        PencilPiece p;
+        long local = 0, total = 0;
+        int L = 0;
+        p.grid = grid_of((long)pos, local, total, L);
+        p.grp = local / L;
+        p.p0 = (int)(local - p.grp * L);
+        p.len = pencil_piece(s, pos, L - p.p0);
+        p.ahead = pos + p.len < s.end && local + p.len < total ? local + p.len : -1;
+        const long long seen = (long long)atomicCAS(&s.pos, (unsigned long long)pos,
+                                                    (unsigned long long)(pos + p.len));
+        if (seen == pos) return p;
+        pos = seen;
+    }
+    return PencilPiece{0, 0, 0, 0, -1};
+}
+
+// One pass along DIR over the job of `a`: every CTA takes an equal contiguous
+// share of the (line group, position) space.
+template <int DIR, typename V, bool UNI, int MODE, bool CLO>
+__global__ void __launch_bounds__(640, 1)
     pencil_rhs_kernel(const __grid_constant__ RhsArgs a, int krk) {
-    using P = PencilLayout<CT>;
     extern __shared__ __align__(16) unsigned char pencil_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    CT* ring = reinterpret_cast<CT*>(pencil_smem) + warp * P::WARP + lane;
-    int L = 0;
-    const long total = pencil_work<DIR>(a, L);
-    const long S = (long)gridDim.x * WPB, s = (long)blockIdx.x * WPB + warp;
-    long pos = total * s / S;
-    const long end = total * (s + 1) / S;
-    while (pos < end) {
-        const long grp = pos / L;
-        const int p0 = (int)(pos - grp * L);
-        const int len = (int)min((long)(L - p0), end - pos);
-        pencil_segment<DIR, CT, UNI, MODE, CLO>(a, krk, ring, grp, p0, len);
-        pos += len;
+    __shared__ PencilShare sh;
+    constexpr size_t G = PencilLayout<V, CLO>::template bytes<MODE>();
+    if (threadIdx.x == 0) {
+        int L = 0;
+        pencil_share(sh, pencil_work<DIR, PencilLayout<V, CLO>::GL>(a, L));
+        pencil_init_bars(pencil_smem + G - 16, G);
+    }
+    __syncthreads();
+    const int tg = threadIdx.x >= 320;
+    const bool lead = threadIdx.x == tg * 320;
+    unsigned phase = 0;
+    for (;;) {
+        if (lead)
+            sh.piece[tg] = pencil_take(sh, [&](long pos, long& local, long& total, int& L) {
+                total = pencil_work<DIR, PencilLayout<V, CLO>::GL>(a, L);
+                local = pos;
+                return 0;
+            });
+        pencil_sync(tg);                   // the piece is known, the last one is out
+        const PencilPiece& p = sh.piece[tg];
+        if (p.len == 0) break;
+        pencil_segment<DIR, V, UNI, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, p);
     }
 }
 
 // The same pass over the grids of a batch: argument table `grids`, and
-// woff[i] the pass's work before grid i (woff[n] the total).  A warp's share
-// may cross grids.
-template <int DIR, int WPB, typename CT, int MODE, bool CLO = false>
-__global__ void __launch_bounds__(WPB * 32, 1)
+// woff[i] the pass's work before grid i (woff[n] the total).  A share may
+// cross grids; each group copies the arguments of its piece's grid (without
+// the tensor maps) to shared memory.
+constexpr int kArgWords = (int)(offsetof(RhsArgs, tma) / 4);
+template <int DIR, typename V, int MODE, bool CLO>
+__global__ void __launch_bounds__(640, 1)
     pencil_batch_kernel(const RhsArgs* __restrict__ grids, const long* __restrict__ woff, int n,
                         int krk) {
-    using P = PencilLayout<CT>;
     extern __shared__ __align__(16) unsigned char pencil_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    CT* ring = reinterpret_cast<CT*>(pencil_smem) + warp * P::WARP + lane;
-    const long total = woff[n];
-    const long S = (long)gridDim.x * WPB, s = (long)blockIdx.x * WPB + warp;
-    long pos = total * s / S;
-    const long end = total * (s + 1) / S;
-    int lo = 0, hi = n;                    // the grid holding pos: woff[i] <= pos < woff[i+1]
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (woff[mid] <= pos) lo = mid; else hi = mid;
+    __shared__ PencilShare sh;
+    __shared__ __align__(64) uint32_t argw[2][(kArgWords + 15) / 16 * 16];
+    constexpr size_t G = PencilLayout<V, CLO>::template bytes<MODE>();
+    if (threadIdx.x == 0) {
+        pencil_share(sh, woff[n]);
+        pencil_init_bars(pencil_smem + G - 16, G);
     }
-    int i = lo;
-    while (pos < end) {
-        while (woff[i + 1] <= pos) ++i;
-        const RhsArgs& a = grids[i];
-        int L = 0;
-        pencil_work<DIR>(a, L);
-        const long local = pos - woff[i];
-        const long grp = local / L;
-        const int p0 = (int)(local - grp * L);
-        const int len = (int)min((long)(L - p0), end - pos);
-        pencil_segment<DIR, CT, true, MODE, CLO>(a, krk, ring, grp, p0, len);
-        pos += len;
-    }
-}
-
-// The x pass, cooperative.  In the other passes a warp's 32 lines are
-// consecutive in x, so the per-lane loads and du stores coalesce; in the x
-// pass they are 32 consecutive y, and per lane every access is a separate
-// L1 transaction (measured: MIO-throttle-bound, 3x the y pass's time in the
-// mixed form).  Here the lanes still own their lines and reconstruct their
-// own faces, but the loads and splits of the next C points of all 32 lines,
-// and the stores of C points of du, are done by the warp together: lane
-// (xi, yi) = (lane % C, lane / C) takes point xi of lines yi + r (32 / C),
-// r < C, so each access covers 32 / C lines x C consecutive x.  A split is
-// then written into the owning lane's ring column, so the ring holds 8 + C
-// slots (a chunk of C faces spans 7 + C stencil points).  C = 4 for the
-// mixed form; C = 2 for FP64, whose larger ring must leave room for 8 warps.
-template <typename CT, int C_>
-struct PencilXLayout {
-    static constexpr int C = C_;                  // points per chunk (and lanes per line row)
-    static constexpr int SLOTS = 8 + C;           // a chunk's 8-point stencils span 7 + C points
-    static constexpr int RS = 10 * 32;
-    static constexpr int RING = SLOTS * RS;       // CT
-    static constexpr int DUS = 5 * C * 32;        // du staging, doubles
-    static constexpr size_t WARP_BYTES = RING * sizeof(CT) + DUS * sizeof(double);
-};
-// chunk of the cooperative x pass: 4 for the mixed form, 2 for FP64 (whose
-// ring is twice as large; 8 warps per CTA then still fit)
-template <typename CT>
-constexpr int pencil_x_chunk() { return sizeof(CT) == 4 ? 4 : 2; }
-
-// One segment of the cooperative x pass (positions p0 .. p0+len-1 of the 32
-// lines of group grp); wbase: the warp's ring and du staging.  CLO: faces
-// next to a CLOSURE x face take the closure rules (uniform across the warp,
-// whose lanes march the same x).
-template <typename CT, bool UNI, int MODE, bool CLO = false>
-__device__ __forceinline__ void pencil_x_segment(const RhsArgs& a, unsigned char* wbase,
-                                                 long grp, int p0, int len) {
-    static_assert(MODE != P_STAGE, "the x pass never applies the stage");
-    constexpr bool ADD = MODE == P_ADD;
-    using P = PencilXLayout<CT, pencil_x_chunk<CT>()>;
-    constexpr int C = P::C, NS = P::SLOTS, LR = 32 / C;   // lines per load round
-    const int lane = threadIdx.x & 31;
-    CT* ringw = reinterpret_cast<CT*>(wbase);                       // [12][10][32]
-    double* dus = reinterpret_cast<double*>(wbase + P::RING * sizeof(CT));   // [5][C][32]
-    CT* ring = ringw + lane;                                        // this lane's column
-    const SplitK<CT> k = {CT(a.eps2), CT(a.hrg), CT(a.c1), CT(a.c3), CT(a.gm1)};
-    const int nyj = a.ey - a.sy, nzj = a.ez - a.sz;
-    const int mlast = a.nx + 7;
-    const size_t vs = (size_t)a.du_pitch * a.du_ly * a.du_lz;
-    const long NL = (long)nyj * nzj;
-    const int xi = lane % C, yi = lane / C;
-    // this lane's own line, and the C lines it loads / stores for
-    const long lo = min(grp * 32 + lane, NL - 1);
-    const bool valid = grp * 32 + lane < NL;
-    const int oy = a.sy + (int)(lo % nyj), oz = a.sz + (int)(lo / nyj);
-    int cy[C], cz[C];
-    bool cv[C];
-#pragma unroll
-    for (int r = 0; r < C; ++r) {
-        const long l = grp * 32 + yi + LR * r;
-        cv[r] = l < NL;
-        const long lc = min(l, NL - 1);
-        cy[r] = a.sy + (int)(lc % nyj);
-        cz[r] = a.sz + (int)(lc / nyj);
-    }
-    // primitives of point x0 + xi of the C lines (x clamped), and their
-    // splits into the owning lanes' ring columns (only xi < cnt)
-    auto coop_load = [&](int x0, double q[C][5]) {
-        const int x = min(x0 + xi, mlast);
-#pragma unroll
-        for (int r = 0; r < C; ++r)
-#pragma unroll
-            for (int f = 0; f < 5; ++f) q[r][f] = ldg_prim(a, f, x, cy[r], cz[r]);
-    };
-    auto coop_split = [&](int x0, int cnt, const double q[C][5]) {
-        if (xi >= cnt) return;
-        const int x = x0 + xi;
-#pragma unroll
-        for (int r = 0; r < C; ++r) {
-            CT out[10];
-            split_point<0, UNI, CT>(a, k, q[r][0], q[r][1], q[r][2], q[r][3], q[r][4], x,
-                                    cy[r], cz[r], out);
-            CT* dst = ringw + (x % NS) * P::RS + yi + LR * r;
-#pragma unroll
-            for (int c = 0; c < 10; ++c) dst[c * 32] = out[c];
-        }
-    };
-    const bool clo = CLO && (a.clo[0] | a.clo[1]);
-    // face value of variable v above point m (stencil from ring slot s0);
-    // the closure test is compiled only into the chunks of the closure zones
-    auto face = [&](int s0, int m, int v, auto cl) -> double {
-        if constexpr (decltype(cl)::value)
-            return pencil_closure_face<CT>(ring, s0, NS, v, m - 3, a.nx, a.clo[0], a.clo[1],
-                                           false);
-        else
-            return face_flux<CT, true>(ring + s0 * P::RS + v * 32, 5 * 32, P::RS, NS - s0,
-                                       NS * P::RS);
-    };
-    const int ms = a.sx + p0;
-    double qb[C][5];
-    for (int p = ms - 4; p < ms + 4; p += C) {   // the first 8 points
-        coop_load(p, qb);
-        coop_split(p, C, qb);
-    }
-    coop_load(ms + 4, qb);              // the first chunk's new points
-    __syncwarp();
-    double fprev[5];
-    {
-        const int s0 = (ms - 4) % NS;
-#pragma unroll
-        for (int v = 0; v < 5; ++v)
-            fprev[v] = face(s0, ms - 1, v, std::integral_constant<bool, CLO>{});
-    }
-    // faces of this lane's line, steps mc .. mc+cnt-1, into the staging
-    auto faces = [&](int mc, int cnt, auto cl) {
-        for (int i = 0; i < cnt; ++i) {
-            const int m = mc + i;
-            const int s0 = (m - 3) % NS;
-            const double J = UNI ? 1.0 : ldg_met(a, 9, m, oy, oz);
-#pragma unroll
-            for (int v = 0; v < 5; ++v) {
-                const double fc = face(s0, m, v, cl);
-                dus[(v * C + i) * 32 + lane] = -J * ((fc - fprev[v]) * a.rhx);
-                fprev[v] = fc;
-            }
-        }
-    };
-    for (int mc = ms; mc < ms + len; mc += C) {
-        const int cnt = min(C, ms + len - mc);
-        coop_split(mc + 4, cnt, qb);     // points mc+4 .. (slots of mc-4-C ..: dead)
-        __syncwarp();
-        if (mc + C < ms + len) coop_load(mc + C + 4, qb);
-        // closure zones: faces m - 3 <= 3 (LAP m <= 6) next to the low x face,
-        // m - 3 >= n - 3 (m >= n) next to the high one
-        if constexpr (CLO) {
-            if (clo && ((a.clo[0] && mc <= 6) || (a.clo[1] && mc + cnt - 1 >= a.nx)))
-                faces(mc, cnt, std::true_type{});
-            else
-                faces(mc, cnt, std::false_type{});
-        } else {
-            faces(mc, cnt, std::false_type{});
-        }
-        __syncwarp();
-        // du of the chunk: point mc + xi of lines yi + LR r
-        if (xi < cnt) {
-            const int x = mc + xi;
-#pragma unroll
-            for (int r = 0; r < C; ++r) {
-                if (!cv[r]) continue;
-                const size_t o = (size_t)(x - a.sx) +
-                                 (size_t)a.du_pitch * ((size_t)(cy[r] - a.sy) +
-                                                       (size_t)a.du_ly * (size_t)(cz[r] - a.sz));
-#pragma unroll
-                for (int v = 0; v < 5; ++v) {
-                    const double r_ = dus[(v * C + xi) * 32 + yi + LR * r];
-                    double* p = a.du + o + v * vs;
-                    *p = ADD ? *p + r_ : r_;
+    __syncthreads();
+    const int tg = threadIdx.x >= 320;
+    const bool lead = threadIdx.x == tg * 320;
+    const RhsArgs& a = *reinterpret_cast<const RhsArgs*>(argw[tg]);
+    unsigned phase = 0;
+    int held = -1;
+    for (;;) {
+        if (lead)
+            sh.piece[tg] = pencil_take(sh, [&](long pos, long& local, long& total, int& L) {
+                int lo = 0, hi = n;        // the grid holding pos: woff[lo] <= pos < woff[lo+1]
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (woff[mid] <= pos) lo = mid; else hi = mid;
                 }
-            }
+                total = pencil_work<DIR, PencilLayout<V, CLO>::GL>(grids[lo], L);
+                local = pos - woff[lo];
+                return lo;
+            });
+        pencil_sync(tg);                   // the piece is known, the last one is out
+        const PencilPiece& p = sh.piece[tg];
+        if (p.len == 0) break;
+        if (held != p.grid) {
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(grids + p.grid);
+            for (int w = threadIdx.x - tg * 320; w < kArgWords; w += 320)
+                argw[tg][w] = __ldg(src + w);
+            held = p.grid;
+            pencil_sync(tg);
         }
-        (void)valid;
-    }
-    __syncwarp();
-}
-
-template <int WPB, typename CT, bool UNI, int MODE, bool CLO = false>
-__global__ void __launch_bounds__(WPB * 32, 1)
-    pencil_x_coop_kernel(const __grid_constant__ RhsArgs a) {
-    extern __shared__ __align__(16) unsigned char pencil_smem[];
-    const int warp = threadIdx.x >> 5;
-    unsigned char* wbase = pencil_smem + warp * PencilXLayout<CT, pencil_x_chunk<CT>()>::WARP_BYTES;
-    int L = 0;
-    const long total = pencil_work<0>(a, L);
-    const long S = (long)gridDim.x * WPB, s = (long)blockIdx.x * WPB + warp;
-    long pos = total * s / S;
-    const long end = total * (s + 1) / S;
-    while (pos < end) {
-        const long grp = pos / L;
-        const int p0 = (int)(pos - grp * L);
-        const int len = (int)min((long)(L - p0), end - pos);
-        pencil_x_segment<CT, UNI, MODE, CLO>(a, wbase, grp, p0, len);
-        pos += len;
+        pencil_segment<DIR, V, true, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, p);
     }
 }
 
-template <int WPB, typename CT, int MODE, bool CLO = false>
-__global__ void __launch_bounds__(WPB * 32, 1)
-    pencil_x_coop_batch_kernel(const RhsArgs* __restrict__ grids, const long* __restrict__ woff,
-                               int n) {
-    extern __shared__ __align__(16) unsigned char pencil_smem[];
-    const int warp = threadIdx.x >> 5;
-    unsigned char* wbase = pencil_smem + warp * PencilXLayout<CT, pencil_x_chunk<CT>()>::WARP_BYTES;
-    const long total = woff[n];
-    const long S = (long)gridDim.x * WPB, s = (long)blockIdx.x * WPB + warp;
-    long pos = total * s / S;
-    const long end = total * (s + 1) / S;
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (woff[mid] <= pos) lo = mid; else hi = mid;
-    }
-    int i = lo;
-    while (pos < end) {
-        while (woff[i + 1] <= pos) ++i;
-        const RhsArgs& a = grids[i];
-        int L = 0;
-        pencil_work<0>(a, L);
-        const long local = pos - woff[i];
-        const long grp = local / L;
-        const int p0 = (int)(local - grp * L);
-        const int len = (int)min((long)(L - p0), end - pos);
-        pencil_x_segment<CT, true, MODE, CLO>(a, wbase, grp, p0, len);
-        pos += len;
-    }
-}
-
-// Launch of a persistent line-pass kernel, one CTA per SM; the dynamic
-// shared memory size is set and the SM count read once per device per kernel.
+// Launch of a line pass of one CTA per SM, but no more than `most`.  The
+// dynamic shared memory size is set and the SM count read once per device per
+// kernel.
 template <typename Kern, typename... Args>
-int pencil_launch(Kern kern, int* blocks, int threads, size_t smem, cudaStream_t st,
+int pencil_launch(Kern kern, int* blocks, int threads, size_t smem, long most, cudaStream_t st,
                   Args... args) {
     int dev = 0;
     WS_CUDA(cudaGetDevice(&dev));
@@ -504,43 +610,48 @@ int pencil_launch(Kern kern, int* blocks, int threads, size_t smem, cudaStream_t
                                      (int)smem));
         blocks[dev] = sms;
     }
-    kern<<<blocks[dev], threads, smem, st>>>(args...);
+    kern<<<(unsigned)std::min<long>(blocks[dev], std::max(1L, most)), threads, smem, st>>>(args...);
     WS_CUDA(cudaGetLastError());
     return WS_OK;
 }
+constexpr long kAllSms = 1L << 40;
 
-template <int WPB, typename CT, bool UNI>
+// work of pass dir over nx x ny x nz cells: groups of gl lines x positions
+inline long pencil_places(long nx, long ny, long nz, int dir, int gl) {
+    const long nl = dir == 0 ? ny * nz : (dir == 1 ? nx * nz : nx * ny);
+    return (nl + gl - 1) / gl * (dir == 0 ? nx : (dir == 1 ? ny : nz));
+}
+
+// Host side of the passes for one value type and metric kind.
+template <typename V, bool UNI>
 struct PencilLauncher {
-    static constexpr size_t SMEM = (size_t)WPB * PencilLayout<CT>::WARP * sizeof(CT);
-    static constexpr int XW = 8;                       // warps of the cooperative x pass
-    static constexpr size_t XSMEM = XW * PencilXLayout<CT, pencil_x_chunk<CT>()>::WARP_BYTES;
-    // the stage pass holds more operands than the other passes: the mixed
-    // form's runs with 12 warps (16 leave 128 registers), the FP64 one with 8
-    static constexpr int SW = sizeof(CT) == 4 ? (WPB > 12 ? 12 : WPB) : (WPB > 8 ? 8 : WPB);
-    static constexpr size_t SSMEM = (size_t)SW * PencilLayout<CT>::WARP * sizeof(CT);
-
-    // one grid (job of a)
+    static constexpr int GL = 32 * LineVal<V>::NL;
+    static constexpr bool MIXED = LineVal<V>::NL > 1;
+    // one grid (job of a); a CTA with fewer than 2 positions to march would
+    // spend itself on prologues
     template <int DIR, int MODE, bool CLO = false>
     static int one(const RhsArgs& a, int krk, cudaStream_t st) {
-        constexpr int W = MODE == P_STAGE ? SW : WPB;
         static int blocks[64] = {0};
-        return pencil_launch(pencil_rhs_kernel<DIR, W, CT, UNI, MODE, CLO>, blocks, W * 32,
-                             MODE == P_STAGE ? SSMEM : SMEM, st, a, krk);
+        return pencil_launch(
+            pencil_rhs_kernel<DIR, V, UNI, MODE, CLO>, blocks, 640,
+            2 * PencilLayout<V, CLO>::template bytes<MODE>(),
+            pencil_places(a.ex - a.sx, a.ey - a.sy, a.ez - a.sz, DIR, GL) / 2, st, a, krk);
     }
-    template <int MODE, bool CLO>
-    static int xcoop(const RhsArgs& a, cudaStream_t st) {
+    // the z pass with the stage update of the mixed form (12 warps: 16 leave
+    // 128 registers)
+    static int lane_stage(const RhsArgs& a, int krk, cudaStream_t st) {
         static int blocks[64] = {0};
-        return pencil_launch(pencil_x_coop_kernel<XW, CT, UNI, MODE, CLO>, blocks, XW * 32,
-                             XSMEM, st, a);
+        return pencil_launch(pencil_lane_kernel<12>, blocks, 384,
+                             12 * LaneLayout::WARP * sizeof(float), kAllSms, st, a, krk);
     }
     // the x and y passes (each pass's closure instance when the grid has a
     // CLOSURE face in its direction)
     static int xy(const RhsArgs& a, bool add_x, cudaStream_t st) {
         int rc;
         if (a.clo[0] | a.clo[1])
-            rc = add_x ? xcoop<P_ADD, true>(a, st) : xcoop<P_STORE, true>(a, st);
+            rc = add_x ? one<0, P_ADD, true>(a, 0, st) : one<0, P_STORE, true>(a, 0, st);
         else
-            rc = add_x ? xcoop<P_ADD, false>(a, st) : xcoop<P_STORE, false>(a, st);
+            rc = add_x ? one<0, P_ADD>(a, 0, st) : one<0, P_STORE>(a, 0, st);
         if (rc) return rc;
         return (a.clo[2] | a.clo[3]) ? one<1, P_ADD, true>(a, 0, st) : one<1, P_ADD>(a, 0, st);
     }
@@ -553,41 +664,44 @@ struct PencilLauncher {
     static int stage(const RhsArgs& a, bool add_x, int krk, cudaStream_t st) {
         if constexpr (UNI) {
             int rc = xy(a, add_x, st);
-            return rc ? rc : one<2, P_STAGE>(a, krk, st);
+            if (rc) return rc;
+            if constexpr (MIXED) return lane_stage(a, krk, st);
+            else return one<2, P_STAGE>(a, krk, st);
         } else {
             return fail(WS_ERR_UNSUPPORTED, "stage update needs Cartesian metrics");
         }
     }
 
-    // a batch: argument table g of n grids, woff = the three passes' work
-    // prefix tables of n + 1 entries each (x, y, z); krk 0: RHS into each du;
-    // clo: some grid has a CLOSURE face
+    // a batch: argument table g of n grids, woff = the passes' work prefix
+    // tables of n + 1 entries each (x, y, z, z in groups of 32 lines); krk 0:
+    // RHS into each du; clo: some grid has a CLOSURE face
     template <int DIR, int MODE, bool CLO = false>
     static int one_batch(const RhsArgs* g, const long* woff, int n, int krk, cudaStream_t st) {
-        constexpr int W = MODE == P_STAGE ? SW : WPB;
         static int blocks[64] = {0};
-        return pencil_launch(pencil_batch_kernel<DIR, W, CT, MODE, CLO>, blocks, W * 32,
-                             MODE == P_STAGE ? SSMEM : SMEM, st, g, woff, n, krk);
+        return pencil_launch(pencil_batch_kernel<DIR, V, MODE, CLO>, blocks, 640,
+                             2 * PencilLayout<V, CLO>::template bytes<MODE>(), kAllSms, st, g,
+                             woff + DIR * (n + 1), n, krk);
     }
-    template <bool CLO>
-    static int xy_batch(const RhsArgs* g, const long* woff, int n, cudaStream_t st) {
+    // the same z pass of the mixed form: with its arguments from global memory
+    // it needs the registers of 8 warps
+    static int lane_stage_batch(const RhsArgs* g, const long* woff, int n, int krk,
+                                cudaStream_t st) {
         static int blocks[64] = {0};
-        int rc = pencil_launch(pencil_x_coop_batch_kernel<XW, CT, P_STORE, CLO>, blocks, XW * 32,
-                               XSMEM, st, g, woff, n);
-        return rc ? rc : one_batch<1, P_ADD, CLO>(g, woff + (n + 1), n, 0, st);
+        return pencil_launch(pencil_lane_batch_kernel<8>, blocks, 256,
+                             8 * LaneLayout::WARP * sizeof(float), kAllSms, st, g,
+                             woff + 3 * (n + 1), n, krk);
     }
     static int batch(const RhsArgs* g, const long* woff, int n, int krk, bool clo,
                      cudaStream_t st) {
-        int rc = clo ? xy_batch<true>(g, woff, n, st) : xy_batch<false>(g, woff, n, st);
+        int rc = clo ? one_batch<0, P_STORE, true>(g, woff, n, 0, st)
+                     : one_batch<0, P_STORE>(g, woff, n, 0, st);
         if (rc) return rc;
-        if (!krk) return one_batch<2, P_ADD>(g, woff + 2 * (n + 1), n, 0, st);
-        // the batched mixed stage pass (arguments read from global memory)
-        // needs the registers of 8 warps per CTA
-        if constexpr (sizeof(CT) == 4 && WPB != 8)
-            return PencilLauncher<8, CT, true>::template one_batch<2, P_STAGE>(
-                g, woff + 2 * (n + 1), n, krk, st);
-        else
-            return one_batch<2, P_STAGE>(g, woff + 2 * (n + 1), n, krk, st);
+        rc = clo ? one_batch<1, P_ADD, true>(g, woff, n, 0, st)
+                 : one_batch<1, P_ADD>(g, woff, n, 0, st);
+        if (rc) return rc;
+        if (!krk) return one_batch<2, P_ADD>(g, woff, n, 0, st);
+        if constexpr (MIXED) return lane_stage_batch(g, woff, n, krk, st);
+        else return one_batch<2, P_STAGE>(g, woff, n, krk, st);
     }
 };
 

@@ -131,23 +131,23 @@ TileCfg tile_cfg(int i);
 int find_tile_cfg(int bx, int by, int threads);   // index or -1
 int default_cfg(int precision, bool stage);       // tuned default shape (stage kernel or plain RHS)
 
-// The RHS as three line passes x, y, z (pencil_impl.cuh), wpb warps per CTA
-// (0: the default), one CTA per SM; CLOSURE faces of the grid (a.clo) run the
-// x and y passes' closure instances.  krk 0: the RHS into
+// The RHS as three line passes x, y, z (pencil_impl.cuh); CLOSURE faces of the
+// grid (a.clo) run the x and y passes' closure instances.  krk 0: the RHS into
 // a.du; krk 1..3: the RHS into a.du, the z pass applying stage krk (a.f_in,
 // a.fn -> a.f_out, primitives to a.p_out).  add_x: a.du already holds terms
 // the RHS adds to (the viscous terms).
-int launch_rhs_pencil(const RhsArgs& a, int precision, bool uniform, int wpb, int krk,
-                      bool add_x, cudaStream_t st);
+int launch_rhs_pencil(const RhsArgs& a, int precision, bool uniform, int krk, bool add_x,
+                      cudaStream_t st);
 // The line passes over a batch: g the argument table of n Cartesian grids
-// (each with its du), woff the x, y and z passes' work prefix tables (n + 1
-// entries each, pencil_pass_work); krk as launch_rhs_pencil (no add_x); clo:
-// some grid has a CLOSURE face (the x and y passes' closure instances).
+// (each with its du), woff the work prefix tables of pencil_pass_work's
+// kWorkTables dirs (n + 1 entries each); krk as launch_rhs_pencil (no add_x);
+// clo: some grid has a CLOSURE face (the x and y passes' closure instances).
 int launch_rhs_pencil_batch(const RhsArgs* g, const long* woff, int n, int precision, int krk,
                             bool clo, cudaStream_t st);
+constexpr int kWorkTables = 4;
 long pencil_pass_work(const ws_grid& g, int dir);
 // Whether a launch with tile selection `tile` runs the line passes: an
-// explicit request (tile_x < 0, threads = 32 x warps per CTA or 0), or the
+// explicit request (tile_x < 0, or a tile shape with scan_z < 0), or the
 // default (all zeros); an explicit fused tile runs the fused kernel.
 bool use_pencil(const ws_grid* g, ws_tile tile);
 
