@@ -195,6 +195,12 @@ RhsArgs make_rhs_args(const ws_grid* g, ws_job job, const ws_field prims[5],
     return a;
 }
 
+void set_own_ghosts(RhsArgs& a, const ws_grid* g) {
+    for (int i = 0; i < 6; ++i)
+        a.gk[i] = g->face_kind[i] == WS_FACE_PERIODIC ? 1
+                  : g->face_kind[i] == WS_FACE_EXTERNAL ? 0 : 2;
+}
+
 int set_rhs_stage(RhsArgs& a, const ws_grid* g, ws_soa f_in, ws_soa fn, ws_soa f_out,
                   const ws_field p_out[6], double dt, int* status) {
     auto same = [](const ws_soa& x, const ws_soa& y) {
@@ -287,7 +293,7 @@ int rhs_enqueue(const ws_grid* g, ws_job job, const ws_field prims[5], const ws_
 // new primitives p_out.
 int rhs_stage_enqueue(const ws_grid* g, const ws_field p_in[6], ws_soa f_in, ws_soa fn,
                       ws_soa f_out, const ws_field p_out[6], double dt, int krk, int* status,
-                      ws_soa dvis, ws_soa du, ws_tile tile, cudaStream_t st) {
+                      ws_soa dvis, ws_soa du, ws_tile tile, bool own_ghosts, cudaStream_t st) {
     if (use_pencil(g, tile)) {
         int rc = check_pencil(g, tile);
         if (rc) return rc;
@@ -297,6 +303,7 @@ int rhs_stage_enqueue(const ws_grid* g, const ws_field p_in[6], ws_soa f_in, ws_
         const ws_field p5[5] = {p_in[0], p_in[1], p_in[2], p_in[3], p_in[5]};
         RhsArgs a = make_rhs_args(g, job, p5, nullptr, du, 0, 1);
         if ((rc = set_rhs_stage(a, g, f_in, fn, f_out, p_out, dt, status))) return rc;
+        if (own_ghosts) set_own_ghosts(a, g);
         return launch_rhs_pencil(a, g->precision, true, krk, dvis.ptr != nullptr, st);
     }
     int cfg = 0;

@@ -221,7 +221,8 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     auto fetch_prims = [&](int k) {
         const int i = k * C + sx;
         if (i < len) {
-            const Pt p = point(ms + 4 + i, sln);
+            const int m = ms + 4 + i;
+            const Pt p = point(UNI ? pencil_source_ahead<DIR>(a, m) : m, sln);
 #pragma unroll
             for (int f = 0; f < 5; ++f)
 #pragma unroll
@@ -429,6 +430,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
             if (i >= plen + 8) continue;
             Pt p;
             p.m = ms - p0 + pp - 4 + i;
+            if (UNI) p.m = pencil_source<DIR>(a, p.m);
 #pragma unroll
             for (int h = 0; h < NL; ++h)
                 fixed((int)g * P::GL + ln + 32 * h, p.c1[h], p.c2[h]);

@@ -26,6 +26,21 @@ struct LaneLayout {
     static constexpr int WARP = 8 * RS;           // one warp's ring
 };
 
+// LAP position whose primitives point m of a line has (RhsArgs::gk); _ahead:
+// of a point past the first four, as the march takes them.
+template <int DIR>
+__device__ __forceinline__ int pencil_source_ahead(const RhsArgs& a, int m) {
+    const int n = DIR == 0 ? a.nx : (DIR == 1 ? a.ny : a.nz);
+    if (m < n + 4) return m;
+    return a.gk[2 * DIR + 1] == 1 ? m - n : a.gk[2 * DIR + 1] == 2 ? n + 3 : m;
+}
+template <int DIR>
+__device__ __forceinline__ int pencil_source(const RhsArgs& a, int m) {
+    const int n = DIR == 0 ? a.nx : (DIR == 1 ? a.ny : a.nz);
+    if (m < 4) return a.gk[2 * DIR] == 1 ? m + n : a.gk[2 * DIR] == 2 ? 4 : m;
+    return pencil_source_ahead<DIR>(a, m);
+}
+
 // work of the pass over the job of `a`: groups of 32 lines x positions
 __device__ __forceinline__ long lane_work(const RhsArgs& a, int& L) {
     L = a.ez - a.sz;
@@ -48,8 +63,9 @@ __device__ __forceinline__ void lane_segment(const RhsArgs& a, int krk, float* r
     if (!valid) l = NL - 1;
     const int x = a.sx + (int)(l % nxj), y = a.sy + (int)(l / nxj);
     auto load = [&](int z, double q[5]) {
+        const int zs = pencil_source<2>(a, z);
 #pragma unroll
-        for (int f = 0; f < 5; ++f) q[f] = ldg_prim(a, f, x, y, z);
+        for (int f = 0; f < 5; ++f) q[f] = ldg_prim(a, f, x, y, zs);
     };
     auto split_into = [&](int z, const double q[5]) {
         float out[10];

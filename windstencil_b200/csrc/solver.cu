@@ -4,8 +4,8 @@
 // Replaces the reference's time loop (src/solver/OCFD_NS_Solver.cpp:64-90)
 // for the Euler system.  The reference's pf/pfn pointer swap becomes two
 // captured graphs (state buffer 0 -> 1 and 1 -> 0), each holding three
-// stages of
-//   ghost fill (d,u,v,w,T,cc) -> fused RHS with the SSP-RK3 stage epilogue,
+// stages of the RHS with the SSP-RK3 stage epilogue (the line passes; with an
+// explicit tile shape a ghost fill and the fused sweep),
 // which writes the stage's conserved state and its primitives into the other
 // primitive buffer.  The reference's shipped loop runs stage 1 only
 // (`KRK <= 1`, :77); all three stage formulas of OCFD_time.cpp:15-65 are used.
@@ -69,19 +69,25 @@ const ws_field* stage_input(const GridState& g, int c, int krk) {
 // Stage krk of the SSP-RK3 step from state buffer c into 1-c; primitives
 // pr[c] -> pr[1-c] (stage 1), pr[1-c] -> pr[c] (stage 2), pr[c] -> pr[1-c]
 // (stage 3).  First half: ghost fill of the stage's input (faces that are
-// not EXTERNAL) and, with viscous terms, their flux pass.
-int enqueue_stage_begin(ws_solver* s, int c, int krk, cudaStream_t st) {
+// not EXTERNAL) and, with viscous terms, their flux pass.  own_ghosts: the
+// line passes take their ghost values from the interior themselves, which
+// leaves a ghost fill of u, v, w, T to the viscous terms (Euler: 0.036 of a
+// stage's 1.92 ms at 600x128x128, one of four launches on a small grid).
+int enqueue_stage_begin(ws_solver* s, int c, int krk, bool own_ghosts, cudaStream_t st) {
     GridState& g = s->s;
     const ws_field* pin = stage_input(g, c, krk);
-    int rc = launch_ghost_fill_prims(&g.g, pin, st);
-    if (rc || !s->viscous) return rc;
     const ws_field p4[4] = {pin[1], pin[2], pin[3], pin[4]};
+    int rc = WS_OK;
+    if (!own_ghosts) rc = launch_ghost_fill_prims(&g.g, pin, st);
+    else if (s->viscous) rc = launch_ghost_fill(&g.g, p4, 4, st);
+    if (rc || !s->viscous) return rc;
     return launch_vis_flux(&g.g, &s->vis, p4, nullptr, s->vis_ws, st);
 }
 
 // Second half: the viscous terms' divergence into du (stored), then the fused
 // RHS with the stage update, which adds them to the inviscid RHS.
-int enqueue_stage_end(ws_solver* s, int c, int krk, double dt, cudaStream_t st) {
+int enqueue_stage_end(ws_solver* s, int c, int krk, double dt, bool own_ghosts,
+                      cudaStream_t st) {
     GridState& g = s->s;
     const ws_field* pin = stage_input(g, c, krk);
     const ws_field* pout = g.pr[krk == 2 ? c : 1 - c];
@@ -92,18 +98,19 @@ int enqueue_stage_end(ws_solver* s, int c, int krk, double dt, cudaStream_t st) 
         dvis = g.du;
     }
     return rhs_stage_enqueue(&g.g, pin, g.f[1 - c], g.f[c], g.f[1 - c], pout, dt, krk,
-                             g.status, dvis, g.du, s->tile, st);
+                             g.status, dvis, g.du, s->tile, own_ghosts, st);
 }
 
-int enqueue_stage(ws_solver* s, int c, int krk, double dt, cudaStream_t st) {
-    int rc = enqueue_stage_begin(s, c, krk, st);
-    return rc ? rc : enqueue_stage_end(s, c, krk, dt, st);
+int enqueue_stage(ws_solver* s, int c, int krk, double dt, bool own_ghosts, cudaStream_t st) {
+    int rc = enqueue_stage_begin(s, c, krk, own_ghosts, st);
+    return rc ? rc : enqueue_stage_end(s, c, krk, dt, own_ghosts, st);
 }
 
 // one SSP-RK3 step from state buffer c into 1-c
 int enqueue_step(ws_solver* s, int c, double dt, cudaStream_t st) {
+    const bool own = use_pencil(&s->s.g, s->tile);
     for (int krk = 1; krk <= 3; ++krk)
-        if (int rc = enqueue_stage(s, c, krk, dt, st)) return rc;
+        if (int rc = enqueue_stage(s, c, krk, dt, own, st)) return rc;
     return WS_OK;
 }
 
@@ -357,7 +364,7 @@ int ws_solver_stage(ws_solver* s, int krk, double dt, ws_stream_t stream) {
         return fail(WS_ERR_UNSUPPORTED, "with viscous terms an EXTERNAL grid stages in two "
                                         "halves (ws_solver_stage_begin / _end) with the "
                                         "fluxes' halo exchange between them");
-    int rc = enqueue_stage(s, s->s.cur, krk, dt, (cudaStream_t)stream);
+    int rc = enqueue_stage(s, s->s.cur, krk, dt, false, (cudaStream_t)stream);
     if (rc) return rc;
     advance_stage(s, krk);
     return WS_OK;
@@ -365,7 +372,7 @@ int ws_solver_stage(ws_solver* s, int krk, double dt, ws_stream_t stream) {
 
 int ws_solver_stage_begin(ws_solver* s, int krk, ws_stream_t stream) {
     if (int rc = check_stage(s, krk, false)) return rc;
-    int rc = enqueue_stage_begin(s, s->s.cur, krk, (cudaStream_t)stream);
+    int rc = enqueue_stage_begin(s, s->s.cur, krk, false, (cudaStream_t)stream);
     if (rc) return rc;
     s->stage_begun = true;
     return WS_OK;
@@ -374,7 +381,7 @@ int ws_solver_stage_begin(ws_solver* s, int krk, ws_stream_t stream) {
 int ws_solver_stage_end(ws_solver* s, int krk, double dt, ws_stream_t stream) {
     if (int rc = check_stage(s, krk, true)) return rc;
     if (!(dt > 0)) return fail(WS_ERR_INVALID, "need dt > 0");
-    int rc = enqueue_stage_end(s, s->s.cur, krk, dt, (cudaStream_t)stream);
+    int rc = enqueue_stage_end(s, s->s.cur, krk, dt, false, (cudaStream_t)stream);
     if (rc) return rc;
     advance_stage(s, krk);
     return WS_OK;

@@ -75,6 +75,10 @@ struct RhsArgs {
     // viscous terms of the stage (ptr NULL: none): du[0..4] added to the
     // inviscid RHS before the update; same SoA shape as fn
     ws_soa dvis;
+    // Line passes: where a ghost point's primitives come from, faces x-, x+,
+    // y-, y+, z-, z+: 0 the ghost layer itself, 1 the wrapped and 2 the clamped
+    // interior point (the values a ghost fill would have put there)
+    int gk[6];
     // TMA staging (tma != 0): per primitive, a map of its LAP array with the
     // (BX+8) x (BY+8) box of a plane and one with the BX x BY centre box.
     // Set only when every box start is 16-byte aligned (even job start x,
@@ -88,6 +92,10 @@ struct RhsArgs {
     CUtensorMap tm_box[5], tm_ctr[5];
 };
 
+// ghost points of `a` from the interior, by the grid's face kinds (EXTERNAL
+// faces keep their layer): a launch that runs the line passes then needs no
+// ghost fill before it
+void set_own_ghosts(RhsArgs& a, const ws_grid* g);
 // fill the epilogue fields of `a` for one stage (WS_ERR_INVALID when the
 // SoA shapes or the p_out pitches differ)
 int set_rhs_stage(RhsArgs& a, const ws_grid* g, ws_soa f_in, ws_soa fn, ws_soa f_out,
@@ -99,10 +107,11 @@ int rhs_ctas(const ws_grid* g, const RhsArgs& a, int cfg, bool stage);
 // new primitives p_out.
 // dvis.ptr may be NULL (no viscous terms).
 // du: the grid's RHS buffer, which the line passes accumulate into (with
-// viscous terms it holds them, and dvis is the same buffer).
+// viscous terms it holds them, and dvis is the same buffer).  own_ghosts (line
+// passes only): see set_own_ghosts.
 int rhs_stage_enqueue(const ws_grid* g, const ws_field p_in[6], ws_soa f_in, ws_soa fn,
                       ws_soa f_out, const ws_field p_out[6], double dt, int krk, int* status,
-                      ws_soa dvis, ws_soa du, ws_tile tile, cudaStream_t st);
+                      ws_soa dvis, ws_soa du, ws_tile tile, bool own_ghosts, cudaStream_t st);
 
 // Viscous terms (viscous.cu): workspace size, parameter check, and du[1..4]
 // += (accumulate) or = the viscous terms (du[0] = 0 when storing) from the
@@ -261,6 +270,7 @@ class BatchRunner {
 
   private:
     int upload_tables(cudaStream_t st);
+    int fill_ghosts(int which, cudaStream_t st);
     std::vector<GridState*> grids_;
     int precision_ = 0, cfg_ = 0, zc_ = 1 << 30, ctas_ = 0;
     bool closure_ = false;          // some grid has CLOSURE faces
