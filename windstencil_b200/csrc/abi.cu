@@ -150,7 +150,7 @@ bool encode_lap_map(CUtensorMap* map, const ws_grid* g, const ws_field& f, int b
 
 RhsArgs make_rhs_args(const ws_grid* g, ws_job job, const ws_field prims[5],
                       const ws_metrics* m, ws_soa du, int cfg, int scan) {
-    const TileCfg c = tile_cfg(cfg);
+    const TileCfg c = tile_cfg(std::max(cfg, 0));
     RhsArgs a{};
     for (int i = 0; i < 5; ++i) {
         a.prim[i] = prims[i].ptr;
@@ -182,9 +182,11 @@ RhsArgs make_rhs_args(const ws_grid* g, ws_job job, const ws_field prims[5],
     a.c3 = (3.0 - g->gamma) / (2.0 * (g->gamma - 1.0));
     a.gm1 = g->gamma - 1.0;
     for (int i = 0; i < 4; ++i) a.clo[i] = g->face_kind[i] == WS_FACE_CLOSURE ? 1 : 0;
+    // cfg < 0: the line passes, which stage without TMA; their calls leave out the
+    // ten map encodings.
     // TMA staging: box starts at x = sx - 4 + k*bx and centres at sx + k*bx
     // are even (16-byte aligned for doubles) when sx is even
-    bool tma = (job.start.x % 2) == 0;
+    bool tma = cfg >= 0 && (job.start.x % 2) == 0;
     for (int i = 0; i < 5 && tma; ++i)
         tma = encode_lap_map(&a.tm_box[i], g, prims[i], c.bx + 8, c.by + 8) &&
               encode_lap_map(&a.tm_ctr[i], g, prims[i], c.bx, c.by);
@@ -275,7 +277,7 @@ int rhs_enqueue(const ws_grid* g, ws_job job, const ws_field prims[5], const ws_
     if (use_pencil(g, tile)) {
         int rc = check_pencil(g, tile);
         if (rc) return rc;
-        const RhsArgs a = make_rhs_args(g, job, prims, m, du, 0, 1);
+        const RhsArgs a = make_rhs_args(g, job, prims, m, du, -1, 1);
         return launch_rhs_pencil(a, g->precision, g->metrics_uniform != 0, 0, false, st);
     }
     int cfg = 0;
@@ -301,7 +303,7 @@ int rhs_stage_enqueue(const ws_grid* g, const ws_field p_in[6], ws_soa f_in, ws_
             return fail(WS_ERR_INVALID, "line passes: du needs the state's shape");
         ws_job job{{4, 4, 4}, {g->nx + 4, g->ny + 4, g->nz + 4}};
         const ws_field p5[5] = {p_in[0], p_in[1], p_in[2], p_in[3], p_in[5]};
-        RhsArgs a = make_rhs_args(g, job, p5, nullptr, du, 0, 1);
+        RhsArgs a = make_rhs_args(g, job, p5, nullptr, du, -1, 1);
         if ((rc = set_rhs_stage(a, g, f_in, fn, f_out, p_out, dt, status))) return rc;
         if (own_ghosts) set_own_ghosts(a, g);
         return launch_rhs_pencil(a, g->precision, true, krk, dvis.ptr != nullptr, st);
