@@ -126,14 +126,15 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // ---- split ------------------------------------------------------------------
 template <typename V>
 struct LineSplitK {
-    V eps2, hrg2, c1, ke;      // eps^2, 0.25/gamma, 2(gamma-1), 1/2 + c3
+    V eps2, c1;                // eps^2, 2(gamma-1)
 };
 
 // F+ in out[0..4], F- in out[5..9] of one point, direction DIR; CART: the
-// unit vector of DIR as metric gradient, else (a1, a2, a3).
+// unit vector of DIR as metric gradient, else (a1, a2, a3).  t0 = 0.25 d / gamma,
+// t0c = t0 c, kc = t0c (1/2 + c3) c.
 template <int DIR, bool CART, typename V>
-__device__ __forceinline__ void line_split(V d, V u, V v, V w, V c, V a1, V a2, V a3,
-                                           const LineSplitK<V>& k, V out[10]) {
+__device__ __forceinline__ void line_split(V t0, V t0c, V kc, V u, V v, V w, V c, V a1, V a2,
+                                           V a3, const LineSplitK<V>& k, V out[10]) {
     V e1, cs, un, k1, k2, k3;          // u.a, c |a|, u.k, k = a / |a|
     if (CART) {
         e1 = un = DIR == 0 ? u : (DIR == 1 ? v : w);
@@ -154,8 +155,6 @@ __device__ __forceinline__ void line_split(V d, V u, V v, V w, V c, V a1, V a2, 
     const V s3 = vsqrt(vfma(e3, e3, k.eps2));
     const V two = vset<V>(2.0);
     const V sg = vadd(s2, s3), ds = vsub(s3, s2);
-    const V t0 = vmul(d, k.hrg2);
-    const V t0c = vmul(t0, c), kc = vmul(t0c, vmul(k.ke, c));
     const V qh = vmul(vset<V>(0.5), vfma(u, u, vfma(v, v, vmul(w, w))));
 #pragma unroll
     for (int h = 0; h < 2; ++h) {      // +, -
@@ -274,6 +273,5 @@ __device__ __forceinline__ double weno_quot(double n, double d) {
     const double e = fma(-d, y, 1.0);
     return vmul(n, fma(y, fma(e, e, e), y));
 }
-__device__ __forceinline__ float2 weno_quot(float2 n, float2 d) { return mul2(n, rcp2(d)); }
 
 }  // namespace ws

@@ -31,8 +31,8 @@
 // per face.  Both signs in a lane would take 112, but their state spilled (10
 // warps at 168 registers: y pass 1.14 ms at 600x128x128, 15 warps at 128: 1.36
 // ms).  Measured at 600x128x128, earlier form -> this one: FP64 x .980 -> .543,
-// y .808 -> .580, z .818 -> .581, z with the stage .948 -> .632 ms; mixed x .487
-// -> .335, y .363 -> .328, z .373 -> .304 ms.  FP64 pipe 65-68% active (ncu);
+// y .808 -> .585, z .818 -> .585, z with the stage .948 -> .632 ms; mixed x .487
+// -> .349, y .363 -> .303, z .373 -> .300 ms.  FP64 pipe 65-68% active (ncu);
 // an FMA with three distinct registers takes it 3 cycles instead of 2, and
 // fixed-latency waits and the exchange take the rest.  du goes through HBM
 // between the passes (~320 B/cell).
@@ -51,15 +51,23 @@ enum PencilMode { P_STORE = 0, P_ADD = 1, P_STAGE = 2 };
 // C points per chunk (the march is unrolled C times, more than the longest
 // lag, so the lagged values rotate through registers).  Ring of four chunks --
 // being written out, marched, ready, being split -- the 8-point prologue in
-// the last 8 slots.  A cell's result goes to the slot of the point just taken
+// the last 8 slots.  A lane's result goes to the slot of the point just taken
 // (OFF = 0), or with CLOSURE faces, which read 7 points of history, 8 slots
 // further back (two more chunks keep it from the splits).
+//
+// The result is the cell's face difference in FP64.  In FP32 (FACE) it is the
+// value of the face above the cell, which the write-out widens and subtracts:
+// both cells at a face then have the same value of it, and du sums to zero over
+// a periodic line to FP64 rounding (differences taken in FP32 left 4e-10 to
+// 6e-9 of sum |du|).  The write-out of a
+// chunk reads the last face of the chunk before too: one more chunk.
 template <typename V, bool CLO>
 struct PencilLayout {
     static constexpr int NL = LineVal<V>::NL, GL = 32 * NL;
+    static constexpr bool FACE = sizeof(typename LineVal<V>::CT) == 4;
     static constexpr int C = 5, NT = 320, HT = NT / 2;   // threads of a group, of one role
-    static constexpr int SLOTS = (CLO ? 6 : 4) * C, OFF = CLO ? 8 : 0;
-    static_assert(SLOTS >= 4 * C + OFF && SLOTS >= 2 * C + 8, "ring");
+    static constexpr int SLOTS = (CLO ? 6 : FACE ? 5 : 4) * C, OFF = CLO ? 8 : 0;
+    static_assert(SLOTS >= 4 * C + OFF + FACE && SLOTS >= 2 * C + 8, "ring");
     // slot stride padded for the x pass, whose lanes write (and read back)
     // neighbouring slots at once; unpadded these would share their banks
     static constexpr int RS = 10 * 32 + 3;               // V per slot
@@ -75,10 +83,10 @@ struct PencilLayout {
     static_assert(sizeof(V) == 8, "one 8-byte value per lane and component");
 };
 
-// 12 x (closure value - central value) of component c (0..4 F+, 5..9 F-) at
-// face f (direction of n cells, CLOSURE flags lo / hi, ydir: the y forms) for
-// line half h, from the lane's ring column's stencil of 8 points starting at
-// slot s0 of `slots`.  Not inlined: only the steps near CLOSURE ends call it,
+// Closure value of component c (0..4 F+, 5..9 F-) at face f (direction of n
+// cells, CLOSURE flags lo / hi, ydir: the y forms) for line half h, from the
+// lane's ring column's stencil of 8 points starting at slot s0 of `slots`; in
+// FP64 12 x (the value - the central one).  Not inlined: only the steps near CLOSURE ends call it,
 // and one copy keeps the march within the instruction cache.
 template <typename V>
 __device__ __noinline__ double pencil_closure_face(const V* col, int s0, int slots, int rs,
@@ -93,6 +101,7 @@ __device__ __noinline__ double pencil_closure_face(const V* col, int s0, int slo
     }
     const double val = minus ? closure_m_arr(s, f, n, lo, hi, ydir)
                              : closure_p_arr(s, f, n, lo, hi, ydir);
+    if (PencilLayout<V, true>::FACE) return val;
     return 12.0 * val - (7.0 * (s[3] + s[4]) - (s[2] + s[5]));
 }
 
@@ -144,7 +153,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     using P = PencilLayout<V, CLO>;
     using CT = typename LineVal<V>::CT;
     constexpr int C = P::C, NL = P::NL, RS = P::RS, HT = P::HT;
-    constexpr bool ADD = MODE != P_STORE;
+    constexpr bool ADD = MODE != P_STORE, FACE = P::FACE;
     const int gt = threadIdx.x - tg * P::NT, lane = gt & 31, warp = gt >> 5;
     const bool minus = warp >= 5;
     V* ring = reinterpret_cast<V*>(smem);
@@ -197,21 +206,33 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         if constexpr (NL == 1) return e[0];
         else return make_float2((float)e[0], (float)e[1]);
     };
-    auto split_into = [&](const V (&q)[5], const Pt& p, int s, int ln) {
-        const LineSplitK<V> k = {vset<V>(a.eps2), vset<V>(0.5 * a.hrg), vset<V>(a.c1),
-                                 vset<V>(0.5 + a.c3)};
-        V g[3], out[10];
+    // the splits of point p with the primitives e into slot s
+    auto split_into = [&](const double (&e)[5][NL], const Pt& p, int s, int ln) {
+        const LineSplitK<V> k = {vset<V>(a.eps2), vset<V>(a.c1)};
+        V q[4], g[3], out[10];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) q[f] = pack(e[f + 1]);
+        // the products that every component has as a factor, rounded once (in
+        // FP32 throughout they were half of the mixed form's error)
+        double t0[NL], t0c[NL], kc[NL];
+#pragma unroll
+        for (int h = 0; h < NL; ++h) {
+            t0[h] = vmul(e[0][h], 0.5 * a.hrg);
+            t0c[h] = vmul(t0[h], e[4][h]);
+            kc[h] = vmul(t0c[h], vmul(0.5 + a.c3, e[4][h]));
+        }
         if (!UNI) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                double e[NL];
+                double m[NL];
 #pragma unroll
                 for (int h = 0; h < NL; ++h)
-                    e[h] = ldg_met(a, 3 * DIR + c, p.x(h), p.y(h), p.z(h));
-                g[c] = pack(e);
+                    m[h] = ldg_met(a, 3 * DIR + c, p.x(h), p.y(h), p.z(h));
+                g[c] = pack(m);
             }
         }
-        line_split<DIR, UNI, V>(q[0], q[1], q[2], q[3], q[4], g[0], g[1], g[2], k, out);
+        line_split<DIR, UNI, V>(pack(t0), pack(t0c), pack(kc), q[0], q[1], q[2], q[3], g[0], g[1],
+                                g[2], k, out);
         V* dst = ring + s * RS + ln;
 #pragma unroll
         for (int c = 0; c < 10; ++c) dst[c * 32] = out[c];
@@ -236,15 +257,12 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         if (i >= len) return;
         Pt p;
         if (!UNI) p = point(ms + 4 + i, sln);
-        V q[5];
+        double e[5][NL];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            double e[NL];
+        for (int f = 0; f < 5; ++f)
 #pragma unroll
-            for (int h = 0; h < NL; ++h) e[h] = *prim_slot(f, h);
-            q[f] = pack(e);
-        }
-        split_into(q, p, base + sx, sln);
+            for (int h = 0; h < NL; ++h) e[f][h] = *prim_slot(f, h);
+        split_into(e, p, base + sx, sln);
     };
 
     // ---- results
@@ -282,7 +300,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         }
         if (ADD) cp_async_commit();
     };
-    const double rh12 = (DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz)) * (1.0 / 12.0);
+    const double rh = (DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz)) * (FACE ? 1.0 : 1.0 / 12.0);
     // result of this thread's point of chunk k at slot `base`
     auto write_cells = [&](int k, int base) {
         const int i = k * C + sx;
@@ -291,6 +309,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         const Pt p = point(ms + i, sln);
         int s = base + sx - P::OFF;
         if (P::OFF > 0 && s < 0) s += P::SLOTS;
+        const int sb = s > 0 ? s - 1 : P::SLOTS - 1;       // FACE: of the face below the cell
 #pragma unroll
         for (int h = 0; h < NL; ++h) {
             if (line0 + sln + 32 * h >= nlines) continue;
@@ -300,9 +319,18 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
 #pragma unroll
             for (int w = 0; w < 5; ++w) {
                 const V* e = ring + s * RS + w * 32 + sln;
-                const double sum = (double)reinterpret_cast<const CT*>(e)[h] +
-                                   (double)reinterpret_cast<const CT*>(e + 160)[h];
-                r[w] = ADD ? fma(-J * rh12, sum, *cell_slot(w, h)) : (-J * rh12) * sum;
+                double sum;
+                if constexpr (FACE) {
+                    const V* b = ring + sb * RS + w * 32 + sln;
+                    sum = (double)(reinterpret_cast<const CT*>(e)[h] +
+                                   reinterpret_cast<const CT*>(e + 160)[h]) -
+                          (double)(reinterpret_cast<const CT*>(b)[h] +
+                                   reinterpret_cast<const CT*>(b + 160)[h]);
+                } else {
+                    sum = (double)reinterpret_cast<const CT*>(e)[h] +
+                          (double)reinterpret_cast<const CT*>(e + 160)[h];
+                }
+                r[w] = ADD ? fma(-J * rh, sum, *cell_slot(w, h)) : (-J * rh) * sum;
             }
             if constexpr (MODE == P_STAGE) {
                 const size_t fo = f_at(p, h);
@@ -324,15 +352,30 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     // ---- faces: this warp's component on the lane's lines
     V* col = ring + warp * 32 + lane;
     WenoLine<V> st{};
-    V G[4]{}, qold{};              // first differences of lags 5..2; last face's value
+    // what the central candidates need.  FP64: first differences of lags 5..2
+    // and the last face's value.  FACE: points of lags 4..2, in H, and the
+    // differences of lags 4 and 3 (the next one is taken again: kept, it spilled)
+    V G[4]{}, H[3]{}, qold{};
+    auto shift = [&]() {
+        if (FACE) {
+            G[1] = G[2]; G[2] = vsub(H[2], H[1]);
+            H[0] = H[1]; H[1] = H[2]; H[2] = st.t;
+        } else {
+            G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
+        }
+    };
     const int nlo = CLO ? a.clo[DIR == 0 ? 0 : 2] : 0, nhi = CLO ? a.clo[DIR == 0 ? 1 : 3] : 0;
     const int ncl = DIR == 0 ? a.nx : a.ny;
-    // takes ring slot s (LAP position m + 4); returns 12 x (the face above m
-    // less its central value) and in cen 12 x the central difference of cell m
+    // takes ring slot s (LAP position m + 4).  FACE: returns the value of the
+    // face above m, as the point t_m below it + (central difference + WENO
+    // correction) / 12.  Else 12 x (that value less its central candidate), and
+    // in cen 12 x the central difference of cell m
     auto push = [&](auto mi, int s, int m, V& cen) -> V {
         constexpr bool MI = decltype(mi)::value;
-        cen = vfms(lkc<V, lk::SEVEN>(), vadd(G[1], G[2]), vadd(G[0], G[3]));
-        G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
+        [[maybe_unused]] const V below = H[0];
+        if (FACE) cen = vfma(vset<V>(6.0), G[2], vsub(G[1], vsub(H[2], H[1])));
+        else cen = vfms(lkc<V, lk::SEVEN>(), vadd(G[1], G[2]), vadd(G[0], G[3]));
+        shift();
         V num, den;
         weno_push<MI>(st, col[s * RS], num, den);
         if constexpr (CLO) {
@@ -347,13 +390,16 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
                 return pack(q);
             }
         }
-        return weno_quot(num, den);
+        if constexpr (FACE)
+            return vfma(vset<V>(1.0 / 12.0), vfma(num, vrcp(den), cen), below);
+        else
+            return weno_quot(num, den);
     };
     auto step = [&](auto mi, int s, int m) {
         V cen;
         const V q = push(mi, s, m, cen);
         const int so = P::OFF == 0 ? s : (s >= P::OFF ? s - P::OFF : s - P::OFF + P::SLOTS);
-        col[so * RS] = vadd(cen, vsub(q, qold));
+        col[so * RS] = FACE ? q : vadd(cen, vsub(q, qold));
         qold = q;
     };
     // the march of one sign: state from the prologue's points, then chunk by
@@ -378,11 +424,12 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
 #pragma unroll
         for (int i = 0; i < 7; ++i) {
             V num, den;
-            G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
+            shift();
             weno_push<MI>(st, col[(P::SLOTS - 8 + i) * RS], num, den);
         }
         V cen;
         qold = push(mi, P::SLOTS - 1, ms - 1, cen);
+        if (FACE) col[(P::SLOTS - 1 - P::OFF) * RS] = qold;
         arrive();
         // the last chunk runs in full: its steps past the segment take what the
         // ring happens to hold and leave results that nobody writes out (a
@@ -438,15 +485,12 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         }
     };
     prologue(grp, p0, len, [&](const Pt& p, int i, int ln) {
-        V q[5];
+        double e[5][NL];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            double e[NL];
+        for (int f = 0; f < 5; ++f)
 #pragma unroll
-            for (int h = 0; h < NL; ++h) e[h] = __ldg(prim_at(f, p, h));
-            q[f] = pack(e);
-        }
-        split_into(q, p, i < 8 ? P::SLOTS - 8 + i : i - 8, ln);
+            for (int h = 0; h < NL; ++h) e[f][h] = __ldg(prim_at(f, p, h));
+        split_into(e, p, i < 8 ? P::SLOTS - 8 + i : i - 8, ln);
         if (i == 0)
 #pragma unroll
             for (int h = 0; h < NL; ++h) lines[ln + 32 * h] = make_int2(p.c1[h], p.c2[h]);
