@@ -199,6 +199,21 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     };
 
     // ---- splits
+    // LAP position that stands for position m of a line (source_ahead: past the
+    // first four).  Past a CLOSURE face the closures take no ghost point but
+    // the first one at the high end, while the central candidates do, and
+    // cancel: the passes read the nearest point there that is taken.
+    const int nlo = CLO ? a.clo[DIR == 0 ? 0 : 2] : 0, nhi = CLO ? a.clo[DIR == 0 ? 1 : 3] : 0;
+    const int ncl = DIR == 0 ? a.nx : a.ny;
+    auto source_ahead = [&](int m) {
+        if (CLO && nhi) m = min(m, ncl + 4);
+        return UNI ? pencil_source_ahead<DIR>(a, m) : m;
+    };
+    auto source = [&](int m) {
+        if (CLO && nlo) m = max(m, 4);
+        if (CLO && nhi) m = min(m, ncl + 4);
+        return UNI ? pencil_source<DIR>(a, m) : m;
+    };
     auto prim_at = [&](int f, const Pt& p, int h) {
         return a.prim[f] + lap_index(p.x(h), p.y(h), p.z(h), a.ppitch[f], a.ny);
     };
@@ -243,7 +258,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         const int i = k * C + sx;
         if (i < len) {
             const int m = ms + 4 + i;
-            const Pt p = point(UNI ? pencil_source_ahead<DIR>(a, m) : m, sln);
+            const Pt p = point(source_ahead(m), sln);
 #pragma unroll
             for (int f = 0; f < 5; ++f)
 #pragma unroll
@@ -256,7 +271,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         cp_async_wait<0>();
         if (i >= len) return;
         Pt p;
-        if (!UNI) p = point(ms + 4 + i, sln);
+        if (!UNI) p = point(source_ahead(ms + 4 + i), sln);
         double e[5][NL];
 #pragma unroll
         for (int f = 0; f < 5; ++f)
@@ -364,8 +379,6 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
             G[0] = G[1]; G[1] = G[2]; G[2] = G[3]; G[3] = st.b;
         }
     };
-    const int nlo = CLO ? a.clo[DIR == 0 ? 0 : 2] : 0, nhi = CLO ? a.clo[DIR == 0 ? 1 : 3] : 0;
-    const int ncl = DIR == 0 ? a.nx : a.ny;
     // takes ring slot s (LAP position m + 4).  FACE: returns the value of the
     // face above m, as the point t_m below it + (central difference + WENO
     // correction) / 12.  Else 12 x (that value less its central candidate), and
@@ -477,7 +490,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
             if (i >= plen + 8) continue;
             Pt p;
             p.m = ms - p0 + pp - 4 + i;
-            if (UNI) p.m = pencil_source<DIR>(a, p.m);
+            p.m = source(p.m);
 #pragma unroll
             for (int h = 0; h < NL; ++h)
                 fixed((int)g * P::GL + ln + 32 * h, p.c1[h], p.c2[h]);
