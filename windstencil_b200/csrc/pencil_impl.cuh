@@ -83,26 +83,81 @@ struct PencilLayout {
     static_assert(sizeof(V) == 8, "one 8-byte value per lane and component");
 };
 
-// Closure value of component c (0..4 F+, 5..9 F-) at face f (direction of n
-// cells, CLOSURE flags lo / hi, ydir: the y forms) for line half h, from the
-// lane's ring column's stencil of 8 points starting at slot s0 of `slots`; in
-// FP64 12 x (the value - the central one).  Not inlined: only the steps near CLOSURE ends call it,
-// and one copy keeps the march within the instruction cache.
+// Whether one sign's value at face f (direction of n cells, CLOSURE flags lo /
+// hi) is a closure: the faces of closure_face(), but for F+ at n - 3.
+__device__ __forceinline__ bool pencil_closes(bool minus, int f, int n, int lo, int hi) {
+    return (lo && f <= 3) || (hi && f >= n - (minus ? 3 : 2));
+}
+
+// One sign's closure value at face f of a line, from the ring column of its
+// component (half h), point m + 4 of the face above m in slot s of `slots`; in
+// FP64 12 x (the value - the central one).  The rules of closure_p_arr and
+// closure_m_arr as one formula on the five points q[0..4] about the face, taken
+// from the other side for F-: candidates on q[2..4], q[1..3], q[0..2] with
+// weights 1 / (12e-6 + S)^2 of those that the face has (`use`), divided out of
+// the sum as products of the others; the third face from a low end (F+) has the
+// reference's product weights, and at the ends the value is linear in two points.
+//
+// Not inlined, and one piece of code for all faces, because a step at a CLOSURE
+// end costs what its instructions take to fetch: with a branch per rule, 15
+// interior steps a face.  Measured at 600x128x128 with walls in x and y, before
+// -> now: FP64 x 679 -> 606, y 1149 -> 769 us; mixed x 417 -> 400, y 702 -> 533.
 template <typename V>
-__device__ __noinline__ double pencil_closure_face(const V* col, int s0, int slots, int rs,
+__device__ __noinline__ double pencil_closure_face(const V* col, int s, int slots, int rs,
                                                    bool minus, int h, int f, int n, int lo,
-                                                   int hi, bool ydir) {
+                                                   int hi) {
     using CT = typename LineVal<V>::CT;
-    double s[8];
+    double q[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const int sk = minus ? s - 1 - k : s - 6 + k;
+        q[k] = (double)reinterpret_cast<const CT*>(col + (sk >= 0 ? sk : sk + slots) * rs)[h];
+    }
+    const int e = hi ? n - f : 99, b = lo ? f : 99;    // faces from either end
+    double val;
+    if (e <= (minus ? 1 : 0) || (b == 0 && !minus)) {
+        const double x = b == 0 && !minus ? q[3] : minus && e == 0 ? q[3] : q[2];
+        const double y = b == 0 && !minus ? x : minus ? (e == 0 ? q[4] : q[3]) : q[1];
+        val = x + (minus ? -0.5 : 0.5) * (x - y);
+    } else {
+        const bool third = !minus && (b == 3 || e == 2);
+        const int use = minus ? (b == 0 ? 4 : b == 1 ? 6 : e == 2 ? 3 : 7)
+                              : (b == 1 ? 1 : b == 2 ? 3 : e == 1 ? 6 : 7);
+        auto ind = [](double t0, double t1) {
+            const double S = w5::E12 + (13 * t0 * t0 + 3 * t1 * t1);
+            return S * S;
+        };
+        double d0 = ind(q[2] - 2 * q[3] + q[4], 3 * q[2] - 4 * q[3] + q[4]);
+        double d1 = ind(q[1] - 2 * q[2] + q[3], q[1] - q[3]);
+        double d2 = ind(q[0] - 2 * q[1] + q[2], q[0] - 4 * q[1] + 3 * q[2]);
+        if (!(use & 1)) d0 = 1.0;
+        if (!(use & 2)) d1 = 1.0;
+        if (!(use & 4)) d2 = 1.0;
+        constexpr double z = w5::E12 * w5::E12;
+        const double a0 = third ? z * z : use & 1 ? d1 * d2 : 0.0;
+        const double a1 = third ? d0 * z : use & 2 ? d0 * d2 : 0.0;
+        const double a2 = third || (use & 4) ? d0 * d1 : 0.0;
+        const double c0 = use & 1 ? 2 * q[2] + 5 * q[3] - q[4] : 0.0;
+        const double c1 = use & 2 ? -q[1] + 5 * q[2] + 2 * q[3] : 0.0;
+        const double c2 = use & 4 ? 2 * q[0] - 7 * q[1] + 11 * q[2] : 0.0;
+        val = (a0 * c0 + a1 * c1 + a2 * c2) / (6.0 * (a0 + a1 + a2));
+    }
+    if (PencilLayout<V, true>::FACE) return val;
+    return 12.0 * val - (7.0 * (q[2] + q[3]) - (q[1] + q[4]));
+}
+// The WENO7 value of F+ at the face three from the high end (FACE), which in the
+// mixed form too is FP64 beside the closure of F-.
+template <typename V>
+__device__ __noinline__ double pencil_weno_face(const V* col, int s, int slots, int rs, int h) {
+    double t[8], num, den;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int sk = s0 + k < slots ? s0 + k : s0 + k - slots;
-        s[k] = (double)reinterpret_cast<const CT*>(col + sk * rs)[h];
+        const int sk = s - 7 + k;
+        t[k] = (double)reinterpret_cast<const typename LineVal<V>::CT*>(
+            col + (sk >= 0 ? sk : sk + slots) * rs)[h];
     }
-    const double val = minus ? closure_m_arr(s, f, n, lo, hi, ydir)
-                             : closure_p_arr(s, f, n, lo, hi, ydir);
-    if (PencilLayout<V, true>::FACE) return val;
-    return 12.0 * val - (7.0 * (s[3] + s[4]) - (s[2] + s[5]));
+    weno7_symbo_nd<false>(t, num, den);
+    return t[3] + num / den;
 }
 
 // Barrier of thread group tg of a CTA.
@@ -393,13 +448,14 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         weno_push<MI>(st, col[s * RS], num, den);
         if constexpr (CLO) {
             const int f = m - 3;
-            if (closure_face(f, ncl, nlo, nhi)) {
-                const int s0 = s >= 7 ? s - 7 : s - 7 + P::SLOTS;
+            const bool weno = FACE && !MI && nhi && f == ncl - 3;
+            if (pencil_closes(MI, f, ncl, nlo, nhi) || weno) {
                 double q[NL];
 #pragma unroll
                 for (int h = 0; h < NL; ++h)
-                    q[h] = pencil_closure_face<V>(col, s0, P::SLOTS, RS, MI, h, f, ncl, nlo, nhi,
-                                                  DIR == 1);
+                    q[h] = weno ? pencil_weno_face<V>(col, s, P::SLOTS, RS, h)
+                                : pencil_closure_face<V>(col, s, P::SLOTS, RS, MI, h, f, ncl, nlo,
+                                                         nhi);
                 return pack(q);
             }
         }
