@@ -36,3 +36,26 @@ def test_du_ignores_closure_ghosts(oracle, cuda, shape, tile, precision):
         out.append(du.cpu().numpy())
     assert np.isfinite(out[0]).all()
     assert np.array_equal(*out)
+
+
+@pytest.mark.parametrize("precision", [ws.FP64, ws.MIXED])
+@pytest.mark.parametrize("tile", [None, (16, 8, 0, 704)])
+def test_first_high_ghost_reaches_one_face(oracle, cuda, tile, precision):
+    """The one ghost point that is read, three faces from the high end in x,
+    reaches the two cells at that face and no other."""
+    shape, faces = (19, 24, 6), (CL, CL, CL, CL, PE, PE)
+    g = ws.Grid(*shape, faces=faces, precision=precision)
+    prims = oracle_prims(oracle, or_grid(*shape, face_kind=faces), wl.fourier_state(*shape, seed=72))
+    out = []
+    for value in (None, np.nan):
+        dev = [to_lap(cuda, g, prims[i]) for i in (0, 1, 2, 3, 5)]
+        if value is not None:
+            for t in dev:
+                t[:, :, g.nx + 4] = value
+        du = ws.soa_tensor(g)
+        ws.du_invis_jacobian3d(g, ws.interior_job(g), *dev, du, tile=tile)
+        out.append(du.cpu().numpy())
+    hit = [g.nx - 4, g.nx - 3]
+    assert np.isnan(out[1][..., hit]).all()
+    rest = [i for i in range(g.nx) if i not in hit]
+    assert np.array_equal(out[0][..., rest], out[1][..., rest])

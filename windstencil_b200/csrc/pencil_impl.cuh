@@ -51,9 +51,7 @@ enum PencilMode { P_STORE = 0, P_ADD = 1, P_STAGE = 2 };
 // C points per chunk (the march is unrolled C times, more than the longest
 // lag, so the lagged values rotate through registers).  Ring of four chunks --
 // being written out, marched, ready, being split -- the 8-point prologue in
-// the last 8 slots.  A lane's result goes to the slot of the point just taken
-// (OFF = 0), or with CLOSURE faces, which read 7 points of history, 8 slots
-// further back (two more chunks keep it from the splits).
+// the last 8 slots.  A lane's result goes to the slot of the point just taken.
 //
 // The result is the cell's face difference in FP64.  In FP32 (FACE) it is the
 // value of the face above the cell, which the write-out widens and subtracts:
@@ -61,13 +59,13 @@ enum PencilMode { P_STORE = 0, P_ADD = 1, P_STAGE = 2 };
 // a periodic line to FP64 rounding (differences taken in FP32 left 4e-10 to
 // 6e-9 of sum |du|).  The write-out of a
 // chunk reads the last face of the chunk before too: one more chunk.
-template <typename V, bool CLO>
+template <typename V>
 struct PencilLayout {
     static constexpr int NL = LineVal<V>::NL, GL = 32 * NL;
     static constexpr bool FACE = sizeof(typename LineVal<V>::CT) == 4;
     static constexpr int C = 5, NT = 320, HT = NT / 2;   // threads of a group, of one role
-    static constexpr int SLOTS = (CLO ? 6 : FACE ? 5 : 4) * C, OFF = CLO ? 8 : 0;
-    static_assert(SLOTS >= 4 * C + OFF + FACE && SLOTS >= 2 * C + 8, "ring");
+    static constexpr int SLOTS = (FACE ? 5 : 4) * C;
+    static_assert(SLOTS >= 4 * C + FACE && SLOTS >= 2 * C + 8, "ring");
     // slot stride padded for the x pass, whose lanes write (and read back)
     // neighbouring slots at once; unpadded these would share their banks
     static constexpr int RS = 10 * 32 + 3;               // V per slot
@@ -83,81 +81,72 @@ struct PencilLayout {
     static_assert(sizeof(V) == 8, "one 8-byte value per lane and component");
 };
 
-// Whether one sign's value at face f (direction of n cells, CLOSURE flags lo /
-// hi) is a closure: the faces of closure_face(), but for F+ at n - 3.
-__device__ __forceinline__ bool pencil_closes(bool minus, int f, int n, int lo, int hi) {
-    return (lo && f <= 3) || (hi && f >= n - (minus ? 3 : 2));
+// A zone: the four cells at a CLOSURE end of a line.  They take five faces, of
+// which only the inner one is a WENO7 face on both sides, and their pieces run
+// apart from the march, which so has no closure in it: values next to a CLOSURE
+// end are FP64 in the mixed form too (kept beside the march's FP32 results they
+// cost it 60% in the x pass), no ghost point is read but the one that the WENO7
+// value three faces from a high end takes, and the ring need not hold the
+// points' history.  With walls in x and y, closures in the march -> zones, x and
+// y passes at 600x128x128: FP64 606 + 770 -> 578 + 662 us, mixed (FP32 closure
+// values) 402 + 537 -> 353 + 406; 480x64x32 mixed 55 + 83 -> 48 + 62.
+constexpr int kZone = 4;
+// Position of the march (of L, in job coordinates) at which a piece from
+// position p0 on ends at the latest: zones are pieces of their own.
+template <int DIR, bool CLO>
+__device__ __forceinline__ int pencil_stop(const RhsArgs& a, int p0, int L) {
+    if constexpr (CLO) {
+        const int n = DIR == 0 ? a.nx : a.ny, s = (DIR == 0 ? a.sx : a.sy) - 4;
+        if (a.clo[2 * DIR] && p0 + s < kZone) return min(kZone - s, L);
+        if (a.clo[2 * DIR + 1] && p0 + s < n - kZone) return min(n - kZone - s, L);
+    }
+    return L;
 }
 
-// One sign's closure value at face f of a line, from the ring column of its
-// component (half h), point m + 4 of the face above m in slot s of `slots`; in
-// FP64 12 x (the value - the central one).  The rules of closure_p_arr and
-// closure_m_arr as one formula on the five points q[0..4] about the face, taken
-// from the other side for F-: candidates on q[2..4], q[1..3], q[0..2] with
-// weights 1 / (12e-6 + S)^2 of those that the face has (`use`), divided out of
-// the sum as products of the others; the third face from a low end (F+) has the
-// reference's product weights, and at the ends the value is linear in two points.
-//
-// Not inlined, and one piece of code for all faces, because a step at a CLOSURE
-// end costs what its instructions take to fetch: with a branch per rule, 15
-// interior steps a face.  Measured at 600x128x128 with walls in x and y, before
-// -> now: FP64 x 679 -> 606, y 1149 -> 769 us; mixed x 417 -> 400, y 702 -> 533.
-template <typename V>
-__device__ __noinline__ double pencil_closure_face(const V* col, int s, int slots, int rs,
-                                                   bool minus, int h, int f, int n, int lo,
-                                                   int hi) {
-    using CT = typename LineVal<V>::CT;
+// One sign's closure value at face f of a line of n cells, at its low (hi
+// false) or high CLOSURE end, from the split fluxes t(i) of the zone's points i
+// (i = 0: cell 0, or cell n - 8).  The rules of closure_p_arr and closure_m_arr
+// as one formula on the five points q[0..4] about the face, taken from the other
+// side for F-: candidates on q[2..4], q[1..3], q[0..2] with weights 1 / (12e-6 +
+// S)^2 of those that the face has (`use`), divided out of the sum as products of
+// the others; the third face from an end (F+) has the reference's product
+// weights, and at the ends the value is linear in two points.  One piece of
+// code for all faces: with a branch per rule, within the march, a face cost as
+// much as 15 others.
+template <typename F>
+__device__ __forceinline__ double pencil_closure(F t, bool minus, int f, int n, bool hi) {
+    const int first = hi ? n - 8 : 0;
     double q[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const int sk = minus ? s - 1 - k : s - 6 + k;
-        q[k] = (double)reinterpret_cast<const CT*>(col + (sk >= 0 ? sk : sk + slots) * rs)[h];
-    }
-    const int e = hi ? n - f : 99, b = lo ? f : 99;    // faces from either end
-    double val;
+    for (int k = 0; k < 5; ++k)          // points past the zone's are not used
+        q[k] = t(min(max((minus ? f + 2 - k : f - 3 + k) - first, 0), 8));
+    const int e = hi ? n - f : 99, b = hi ? 99 : f;    // faces from the end
     if (e <= (minus ? 1 : 0) || (b == 0 && !minus)) {
-        const double x = b == 0 && !minus ? q[3] : minus && e == 0 ? q[3] : q[2];
-        const double y = b == 0 && !minus ? x : minus ? (e == 0 ? q[4] : q[3]) : q[1];
-        val = x + (minus ? -0.5 : 0.5) * (x - y);
-    } else {
-        const bool third = !minus && (b == 3 || e == 2);
-        const int use = minus ? (b == 0 ? 4 : b == 1 ? 6 : e == 2 ? 3 : 7)
-                              : (b == 1 ? 1 : b == 2 ? 3 : e == 1 ? 6 : 7);
-        auto ind = [](double t0, double t1) {
-            const double S = w5::E12 + (13 * t0 * t0 + 3 * t1 * t1);
-            return S * S;
-        };
-        double d0 = ind(q[2] - 2 * q[3] + q[4], 3 * q[2] - 4 * q[3] + q[4]);
-        double d1 = ind(q[1] - 2 * q[2] + q[3], q[1] - q[3]);
-        double d2 = ind(q[0] - 2 * q[1] + q[2], q[0] - 4 * q[1] + 3 * q[2]);
-        if (!(use & 1)) d0 = 1.0;
-        if (!(use & 2)) d1 = 1.0;
-        if (!(use & 4)) d2 = 1.0;
-        constexpr double z = w5::E12 * w5::E12;
-        const double a0 = third ? z * z : use & 1 ? d1 * d2 : 0.0;
-        const double a1 = third ? d0 * z : use & 2 ? d0 * d2 : 0.0;
-        const double a2 = third || (use & 4) ? d0 * d1 : 0.0;
-        const double c0 = use & 1 ? 2 * q[2] + 5 * q[3] - q[4] : 0.0;
-        const double c1 = use & 2 ? -q[1] + 5 * q[2] + 2 * q[3] : 0.0;
-        const double c2 = use & 4 ? 2 * q[0] - 7 * q[1] + 11 * q[2] : 0.0;
-        val = (a0 * c0 + a1 * c1 + a2 * c2) / (6.0 * (a0 + a1 + a2));
+        const double x = b == 0 ? q[3] : minus && e == 0 ? q[3] : q[2];
+        const double y = b == 0 ? x : minus ? (e == 0 ? q[4] : q[3]) : q[1];
+        return x + (minus ? -0.5 : 0.5) * (x - y);
     }
-    if (PencilLayout<V, true>::FACE) return val;
-    return 12.0 * val - (7.0 * (q[2] + q[3]) - (q[1] + q[4]));
-}
-// The WENO7 value of F+ at the face three from the high end (FACE), which in the
-// mixed form too is FP64 beside the closure of F-.
-template <typename V>
-__device__ __noinline__ double pencil_weno_face(const V* col, int s, int slots, int rs, int h) {
-    double t[8], num, den;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int sk = s - 7 + k;
-        t[k] = (double)reinterpret_cast<const typename LineVal<V>::CT*>(
-            col + (sk >= 0 ? sk : sk + slots) * rs)[h];
-    }
-    weno7_symbo_nd<false>(t, num, den);
-    return t[3] + num / den;
+    const bool third = !minus && (b == 3 || e == 2);
+    const int use = minus ? (b == 0 ? 4 : b == 1 ? 6 : e == 2 ? 3 : 7)
+                          : (b == 1 ? 1 : b == 2 ? 3 : e == 1 ? 6 : 7);
+    auto ind = [](double t0, double t1) {
+        const double S = w5::E12 + (13 * t0 * t0 + 3 * t1 * t1);
+        return S * S;
+    };
+    double d0 = ind(q[2] - 2 * q[3] + q[4], 3 * q[2] - 4 * q[3] + q[4]);
+    double d1 = ind(q[1] - 2 * q[2] + q[3], q[1] - q[3]);
+    double d2 = ind(q[0] - 2 * q[1] + q[2], q[0] - 4 * q[1] + 3 * q[2]);
+    if (!(use & 1)) d0 = 1.0;
+    if (!(use & 2)) d1 = 1.0;
+    if (!(use & 4)) d2 = 1.0;
+    constexpr double z = w5::E12 * w5::E12;
+    const double a0 = third ? z * z : use & 1 ? d1 * d2 : 0.0;
+    const double a1 = third ? d0 * z : use & 2 ? d0 * d2 : 0.0;
+    const double a2 = third || (use & 4) ? d0 * d1 : 0.0;
+    const double c0 = use & 1 ? 2 * q[2] + 5 * q[3] - q[4] : 0.0;
+    const double c1 = use & 2 ? -q[1] + 5 * q[2] + 2 * q[3] : 0.0;
+    const double c2 = use & 4 ? 2 * q[0] - 7 * q[1] + 11 * q[2] : 0.0;
+    return (a0 * c0 + a1 * c1 + a2 * c2) / (6.0 * (a0 + a1 + a2));
 }
 
 // Barrier of thread group tg of a CTA.
@@ -193,9 +182,7 @@ struct PencilPiece {
 };
 
 // One piece of pass DIR (0 x, 1 y, 2 z) over the job of `a`, by thread group
-// tg of a CTA.  CLO: faces next to a
-// CLOSURE face of the direction take the closure rules (the lines of a group
-// march the same position, so the test is uniform).
+// tg of a CTA.  CLO: pieces at CLOSURE ends of the direction are zones.
 template <int DIR, typename V, bool UNI, int MODE, bool CLO>
 __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsigned char* smem,
                                                int tg, unsigned& phase,
@@ -205,7 +192,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     static_assert(MODE != P_STAGE || (DIR == 2 && UNI && LineVal<V>::NL == 1),
                   "stage update: z pass, Cartesian, FP64");
     static_assert(!CLO || DIR != 2, "closure faces: x and y passes");
-    using P = PencilLayout<V, CLO>;
+    using P = PencilLayout<V>;
     using CT = typename LineVal<V>::CT;
     constexpr int C = P::C, NL = P::NL, RS = P::RS, HT = P::HT;
     constexpr bool ADD = MODE != P_STORE, FACE = P::FACE;
@@ -254,21 +241,6 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     };
 
     // ---- splits
-    // LAP position that stands for position m of a line (source_ahead: past the
-    // first four).  Past a CLOSURE face the closures take no ghost point but
-    // the first one at the high end, while the central candidates do, and
-    // cancel: the passes read the nearest point there that is taken.
-    const int nlo = CLO ? a.clo[DIR == 0 ? 0 : 2] : 0, nhi = CLO ? a.clo[DIR == 0 ? 1 : 3] : 0;
-    const int ncl = DIR == 0 ? a.nx : a.ny;
-    auto source_ahead = [&](int m) {
-        if (CLO && nhi) m = min(m, ncl + 4);
-        return UNI ? pencil_source_ahead<DIR>(a, m) : m;
-    };
-    auto source = [&](int m) {
-        if (CLO && nlo) m = max(m, 4);
-        if (CLO && nhi) m = min(m, ncl + 4);
-        return UNI ? pencil_source<DIR>(a, m) : m;
-    };
     auto prim_at = [&](int f, const Pt& p, int h) {
         return a.prim[f] + lap_index(p.x(h), p.y(h), p.z(h), a.ppitch[f], a.ny);
     };
@@ -313,7 +285,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         const int i = k * C + sx;
         if (i < len) {
             const int m = ms + 4 + i;
-            const Pt p = point(source_ahead(m), sln);
+            const Pt p = point(UNI ? pencil_source_ahead<DIR>(a, m) : m, sln);
 #pragma unroll
             for (int f = 0; f < 5; ++f)
 #pragma unroll
@@ -326,7 +298,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         cp_async_wait<0>();
         if (i >= len) return;
         Pt p;
-        if (!UNI) p = point(source_ahead(ms + 4 + i), sln);
+        if (!UNI) p = point(ms + 4 + i, sln);
         double e[5][NL];
 #pragma unroll
         for (int f = 0; f < 5; ++f)
@@ -377,8 +349,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         if (ADD) cp_async_wait<0>();
         if (i >= len) return;
         const Pt p = point(ms + i, sln);
-        int s = base + sx - P::OFF;
-        if (P::OFF > 0 && s < 0) s += P::SLOTS;
+        const int s = base + sx;
         const int sb = s > 0 ? s - 1 : P::SLOTS - 1;       // FACE: of the face below the cell
 #pragma unroll
         for (int h = 0; h < NL; ++h) {
@@ -438,7 +409,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
     // face above m, as the point t_m below it + (central difference + WENO
     // correction) / 12.  Else 12 x (that value less its central candidate), and
     // in cen 12 x the central difference of cell m
-    auto push = [&](auto mi, int s, int m, V& cen) -> V {
+    auto push = [&](auto mi, int s, V& cen) -> V {
         constexpr bool MI = decltype(mi)::value;
         [[maybe_unused]] const V below = H[0];
         if (FACE) cen = vfma(vset<V>(6.0), G[2], vsub(G[1], vsub(H[2], H[1])));
@@ -446,30 +417,29 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         shift();
         V num, den;
         weno_push<MI>(st, col[s * RS], num, den);
-        if constexpr (CLO) {
-            const int f = m - 3;
-            const bool weno = FACE && !MI && nhi && f == ncl - 3;
-            if (pencil_closes(MI, f, ncl, nlo, nhi) || weno) {
-                double q[NL];
-#pragma unroll
-                for (int h = 0; h < NL; ++h)
-                    q[h] = weno ? pencil_weno_face<V>(col, s, P::SLOTS, RS, h)
-                                : pencil_closure_face<V>(col, s, P::SLOTS, RS, MI, h, f, ncl, nlo,
-                                                         nhi);
-                return pack(q);
-            }
-        }
         if constexpr (FACE)
             return vfma(vset<V>(1.0 / 12.0), vfma(num, vrcp(den), cen), below);
         else
             return weno_quot(num, den);
     };
-    auto step = [&](auto mi, int s, int m) {
+    auto step = [&](auto mi, int s) {
         V cen;
-        const V q = push(mi, s, m, cen);
-        const int so = P::OFF == 0 ? s : (s >= P::OFF ? s - P::OFF : s - P::OFF + P::SLOTS);
-        col[so * RS] = FACE ? q : vadd(cen, vsub(q, qold));
+        const V q = push(mi, s, cen);
+        col[s * RS] = FACE ? q : vadd(cen, vsub(q, qold));
         qold = q;
+    };
+    // state from the eight points in ring slots s0 on; the face value between
+    // the fourth and fifth.  The first seven only fill the state (nothing of
+    // their faces is used, so it is not computed)
+    auto first_face = [&](auto mi, int s0) -> V {
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            V num, den;
+            shift();
+            weno_push<decltype(mi)::value>(st, col[(s0 + i) * RS], num, den);
+        }
+        V cen;
+        return push(mi, s0 + 7, cen);
     };
     // the march of one sign: state from the prologue's points, then chunk by
     // chunk with the exchange after each
@@ -488,17 +458,8 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         constexpr bool MI = decltype(mi)::value;
         if (!MI) fetch_prims(2);
         else fetch_cells(0);
-        // the first seven points only fill the state (nothing of their faces
-        // is used, so it is not computed); the eighth gives the first face
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            V num, den;
-            shift();
-            weno_push<MI>(st, col[(P::SLOTS - 8 + i) * RS], num, den);
-        }
-        V cen;
-        qold = push(mi, P::SLOTS - 1, ms - 1, cen);
-        if (FACE) col[(P::SLOTS - 1 - P::OFF) * RS] = qold;
+        qold = first_face(mi, P::SLOTS - 8);
+        if (FACE) col[(P::SLOTS - 1) * RS] = qold;
         arrive();
         // the last chunk runs in full: its steps past the segment take what the
         // ring happens to hold and leave results that nobody writes out (a
@@ -508,7 +469,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
 #pragma unroll 1
         for (int k = 0; k < nch; ++k) {
 #pragma unroll
-            for (int i = 0; i < C; ++i) step(mi, base + i, ms + k * C + i);
+            for (int i = 0; i < C; ++i) step(mi, base + i);
             await_last();
             if (!MI) {
                 const int s = base + 2 * C;
@@ -546,20 +507,94 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
             if (i >= plen + 8) continue;
             Pt p;
             p.m = ms - p0 + pp - 4 + i;
-            p.m = source(p.m);
+            if (UNI) p.m = pencil_source<DIR>(a, p.m);
 #pragma unroll
             for (int h = 0; h < NL; ++h)
                 fixed((int)g * P::GL + ln + 32 * h, p.c1[h], p.c2[h]);
             f(p, i, ln);
         }
     };
-    prologue(grp, p0, len, [&](const Pt& p, int i, int ln) {
+    auto split_at = [&](const Pt& p, int s, int ln) {
         double e[5][NL];
 #pragma unroll
         for (int f = 0; f < 5; ++f)
 #pragma unroll
             for (int h = 0; h < NL; ++h) e[f][h] = __ldg(prim_at(f, p, h));
-        split_into(e, p, i < 8 ? P::SLOTS - 8 + i : i - 8, ln);
+        split_into(e, p, s, ln);
+    };
+    if constexpr (CLO) {
+        // ---- a zone: the splits of its points (nine at the high end, whose F+
+        // takes the first ghost point), the five faces' values, the cells
+        const int n = DIR == 0 ? a.nx : a.ny;
+        const bool hi = a.clo[2 * DIR + 1] && ms - 4 >= n - kZone;
+        if (hi || (a.clo[2 * DIR] && ms - 4 < kZone)) {
+            const int first = hi ? n - 8 : 0, f0 = hi ? n - kZone : 0, np = hi ? 9 : 8;
+            for (int t = gt; t < np * 32; t += P::NT) {
+                const int i = DIR == 0 ? t % np : t >> 5, ln = DIR == 0 ? t / np : lane;
+                Pt p;
+                p.m = first + i + 4;
+                if (UNI) p.m = pencil_source<DIR>(a, p.m);
+#pragma unroll
+                for (int h = 0; h < NL; ++h)
+                    fixed((int)grp * P::GL + ln + 32 * h, p.c1[h], p.c2[h]);
+                split_at(p, i, ln);
+            }
+            pencil_sync(tg);
+            // face f0 + j of half h, FP64 (in the FP64 form 12 x), in slot 9 + j NL + h
+            static_assert(9 + 5 * NL <= P::SLOTS, "zone's values");
+            auto val = [&](int j, int h, int c, int ln) -> double* {
+                return reinterpret_cast<double*>(ring + (9 + j * NL + h) * RS + c * 32 + ln);
+            };
+            const int inner = hi ? 0 : 4;
+            const V q = minus ? first_face(std::true_type{}, 0) : first_face(std::false_type{}, 0);
+#pragma unroll 1
+            for (int jh = 0; jh < 5 * NL; ++jh) {
+                const int j = jh / NL, h = jh - j * NL;
+                auto t = [&](int i) { return (double)reinterpret_cast<const CT*>(col + i * RS)[h]; };
+                double v;
+                if (j == inner) {
+                    v = (double)reinterpret_cast<const CT*>(&q)[h];
+                    if (!FACE) v += 7.0 * (t(3) + t(4)) - (t(2) + t(5));
+                } else {
+                    if (hi && j == 1 && !minus) {      // F+ three from the end: WENO7
+                        double x[8], num, den;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) x[k] = t(k + 1);
+                        weno7_symbo_nd<false>(x, num, den);
+                        v = x[3] + num / den;
+                    } else {
+                        v = pencil_closure(t, minus, f0 + j, n, hi);
+                    }
+                    if (!FACE) v *= 12.0;
+                }
+                *val(j, h, warp, lane) = v;
+            }
+            pencil_sync(tg);
+            for (int t = gt; t < kZone * P::GL; t += P::NT) {
+                const int j = DIR == 0 ? t % kZone : t / P::GL, l = DIR == 0 ? t / kZone : t % P::GL;
+                const int m = f0 + j + 4, h = l >> 5, ln = l & 31;
+                if (m < ms || m >= ms + len || line0 + l >= nlines) continue;
+                Pt p;
+                p.m = m;
+                fixed(line0 + l, p.c1[0], p.c2[0]);
+                const double k = -(UNI ? 1.0 : ldg_met(a, 9, p.x(0), p.y(0), p.z(0))) * rh;
+                double* du = a.du + du_at(p, 0);
+#pragma unroll
+                for (int w = 0; w < 5; ++w) {
+                    auto sum = [&](int i) -> double {
+                        const double x = *val(i, h, w, ln), y = *val(i, h, w + 5, ln);
+                        // the march's sum at the face that it shares
+                        return FACE && i == inner ? (double)((CT)x + (CT)y) : x + y;
+                    };
+                    const double d = sum(j + 1) - sum(j);
+                    du[w * vs] = ADD ? fma(k, d, du[w * vs]) : k * d;
+                }
+            }
+            return;
+        }
+    }
+    prologue(grp, p0, len, [&](const Pt& p, int i, int ln) {
+        split_at(p, i < 8 ? P::SLOTS - 8 + i : i - 8, ln);
         if (i == 0)
 #pragma unroll
             for (int h = 0; h < NL; ++h) lines[ln + 32 * h] = make_int2(p.c1[h], p.c2[h]);
@@ -608,9 +643,9 @@ __device__ __forceinline__ void pencil_share(PencilShare& s, long total) {
 }
 // The next piece of the share: grid_of(pos, local, total, L) gives the grid of
 // a position, the place within it, its number of places and the march length
-// of its lines.
-template <typename F>
-__device__ __forceinline__ PencilPiece pencil_take(PencilShare& s, F grid_of) {
+// of its lines; stop_of(grid, p0, L) the grid's pencil_stop.
+template <typename F, typename S>
+__device__ __forceinline__ PencilPiece pencil_take(PencilShare& s, F grid_of, S stop_of) {
     long long pos = (long long)*reinterpret_cast<volatile unsigned long long*>(&s.pos);
     while (pos < s.end) {
         PencilPiece p;
@@ -619,7 +654,7 @@ __device__ __forceinline__ PencilPiece pencil_take(PencilShare& s, F grid_of) {
         p.grid = grid_of((long)pos, local, total, L);
         p.grp = local / L;
         p.p0 = (int)(local - p.grp * L);
-        p.len = pencil_piece(s, pos, L - p.p0);
+        p.len = pencil_piece(s, pos, stop_of(p.grid, p.p0, L) - p.p0);
         p.ahead = pos + p.len < s.end && local + p.len < total ? local + p.len : -1;
         const long long seen = (long long)atomicCAS(&s.pos, (unsigned long long)pos,
                                                     (unsigned long long)(pos + p.len));
@@ -636,10 +671,10 @@ __global__ void __launch_bounds__(640, 1)
     pencil_rhs_kernel(const __grid_constant__ RhsArgs a, int krk) {
     extern __shared__ __align__(16) unsigned char pencil_smem[];
     __shared__ PencilShare sh;
-    constexpr size_t G = PencilLayout<V, CLO>::template bytes<MODE>();
+    constexpr size_t G = PencilLayout<V>::template bytes<MODE>();
     if (threadIdx.x == 0) {
         int L = 0;
-        pencil_share(sh, pencil_work<DIR, PencilLayout<V, CLO>::GL>(a, L));
+        pencil_share(sh, pencil_work<DIR, PencilLayout<V>::GL>(a, L));
         pencil_init_bars(pencil_smem + G - 16, G);
     }
     __syncthreads();
@@ -649,10 +684,10 @@ __global__ void __launch_bounds__(640, 1)
     for (;;) {
         if (lead)
             sh.piece[tg] = pencil_take(sh, [&](long pos, long& local, long& total, int& L) {
-                total = pencil_work<DIR, PencilLayout<V, CLO>::GL>(a, L);
+                total = pencil_work<DIR, PencilLayout<V>::GL>(a, L);
                 local = pos;
                 return 0;
-            });
+            }, [&](int, int p0, int L) { return pencil_stop<DIR, CLO>(a, p0, L); });
         pencil_sync(tg);                   // the piece is known, the last one is out
         const PencilPiece& p = sh.piece[tg];
         if (p.len == 0) break;
@@ -672,7 +707,7 @@ __global__ void __launch_bounds__(640, 1)
     extern __shared__ __align__(16) unsigned char pencil_smem[];
     __shared__ PencilShare sh;
     __shared__ __align__(64) uint32_t argw[2][(kArgWords + 15) / 16 * 16];
-    constexpr size_t G = PencilLayout<V, CLO>::template bytes<MODE>();
+    constexpr size_t G = PencilLayout<V>::template bytes<MODE>();
     if (threadIdx.x == 0) {
         pencil_share(sh, woff[n]);
         pencil_init_bars(pencil_smem + G - 16, G);
@@ -691,10 +726,10 @@ __global__ void __launch_bounds__(640, 1)
                     const int mid = (lo + hi) >> 1;
                     if (woff[mid] <= pos) lo = mid; else hi = mid;
                 }
-                total = pencil_work<DIR, PencilLayout<V, CLO>::GL>(grids[lo], L);
+                total = pencil_work<DIR, PencilLayout<V>::GL>(grids[lo], L);
                 local = pos - woff[lo];
                 return lo;
-            });
+            }, [&](int grid, int p0, int L) { return pencil_stop<DIR, CLO>(grids[grid], p0, L); });
         pencil_sync(tg);                   // the piece is known, the last one is out
         const PencilPiece& p = sh.piece[tg];
         if (p.len == 0) break;
@@ -749,7 +784,7 @@ struct PencilLauncher {
         static int blocks[64] = {0};
         return pencil_launch(
             pencil_rhs_kernel<DIR, V, UNI, MODE, CLO>, blocks, 640,
-            2 * PencilLayout<V, CLO>::template bytes<MODE>(),
+            2 * PencilLayout<V>::template bytes<MODE>(),
             pencil_places(a.ex - a.sx, a.ey - a.sy, a.ez - a.sz, DIR, GL) / 2, st, a, krk);
     }
     // the z pass with the stage update of the mixed form (12 warps: 16 leave
@@ -794,7 +829,7 @@ struct PencilLauncher {
     static int one_batch(const RhsArgs* g, const long* woff, int n, int krk, cudaStream_t st) {
         static int blocks[64] = {0};
         return pencil_launch(pencil_batch_kernel<DIR, V, MODE, CLO>, blocks, 640,
-                             2 * PencilLayout<V, CLO>::template bytes<MODE>(), kAllSms, st, g,
+                             2 * PencilLayout<V>::template bytes<MODE>(), kAllSms, st, g,
                              woff + DIR * (n + 1), n, krk);
     }
     // the same z pass of the mixed form: with its arguments from global memory
