@@ -149,9 +149,9 @@ WS_API int  ws_last_error(char* buf, size_t n);
  * (a multiple of 32). */
 WS_API uint32_t ws_lap_pitch(uint32_t nx);
 /* Device-side errors of the launches that carry no per-grid status word
- * (the drop-in RHS entry points): bit value 2 = a staging wait of the fused
- * RHS gave up (bounded wait on its TMA copies) and the launch stopped early,
- * leaving du incomplete.  Reads and clears the word of the current device;
+ * (the drop-in RHS entry points): bit value 2 = a bounded wait gave up (the
+ * line passes' on the warps of a thread group, the tile sweep's on its TMA
+ * copies) and its CTA stopped early, leaving du incomplete.  Reads and clears the word of the current device;
  * synchronises `stream`.  The solver, batches and server report the same bit
  * in their own status words (WS_ERR_TIMEOUT). */
 WS_API int ws_device_error(int* flags, ws_stream_t stream);
@@ -368,8 +368,8 @@ WS_API int  ws_solver_stage_end(ws_solver* s, int krk, double dt, ws_stream_t st
 /* The four viscous flux fields of direction `axis` (Ev1..4, LAP) in the
  * solver's workspace; WS_ERR_INVALID without viscous terms. */
 WS_API int  ws_solver_stage_flux_fields(ws_solver* s, int axis, ws_field ev_axis[4]);
-/* Device status word: 0, WS_ERR_NONFINITE, or WS_ERR_TIMEOUT (a staging
- * wait of the fused RHS gave up); synchronises `stream`. */
+/* Device status word: 0, WS_ERR_NONFINITE, or WS_ERR_TIMEOUT (a bounded wait
+ * of the RHS gave up); synchronises `stream`. */
 WS_API int  ws_solver_status(ws_solver* s, int* status, ws_stream_t stream);
 WS_API int  ws_solver_set_tile(ws_solver* s, ws_tile tile);
 /* Current state to / from a restart file (d, u, v, w, T from / to the

@@ -237,7 +237,7 @@ def ghost_fill(g: Grid, fields, stream=None) -> None:
 
 def device_error(stream=None) -> int:
     """Read and clear the device error word of the launches without a
-    per-grid status (ws_device_error): 2 = a staging wait gave up."""
+    per-grid status (ws_device_error): 2 = a bounded wait gave up."""
     v = C.c_int()
     check(load().ws_device_error(C.byref(v), _stream(stream)))
     return v.value

@@ -193,7 +193,7 @@ RhsArgs make_rhs_args(const ws_grid* g, ws_job job, const ws_field prims[5],
     a.tma = tma ? 1 : 0;
     a.status = device_error_word();     // the stage epilogue sets the grid's own
     const char* hold = std::getenv("WS_TEST_STAGE_WAIT");
-    a.hold_polls = hold ? std::max(0, std::atoi(hold)) : 0;
+    a.hold_polls = hold ? std::min(std::max(0, std::atoi(hold)), 1 << 22) : 0;
     return a;
 }
 

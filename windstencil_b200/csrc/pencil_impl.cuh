@@ -158,10 +158,12 @@ __device__ __forceinline__ void pencil_sync(int tg) {
 __device__ __forceinline__ void pencil_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void pencil_init_bars(unsigned char* first, size_t stride) {
+// hold (the failure path's test): an arrival more than ever comes, so that every
+// wait runs out.
+__device__ __forceinline__ void pencil_init_bars(unsigned char* first, size_t stride, bool hold) {
     for (int g = 0; g < 2; ++g)
         for (int b = 0; b < 2; ++b)
-            mbar_init(reinterpret_cast<uint64_t*>(first + g * stride) + b, 10);
+            mbar_init(reinterpret_cast<uint64_t*>(first + g * stride) + b, hold ? 11 : 10);
 }
 
 // March length and work of pass DIR over the job of `a`: line groups of GL
@@ -181,11 +183,26 @@ struct PencilPiece {
     long grp, ahead;
 };
 
+// Waits for the phase of parity `parity`; false when it gives up, after `hold`
+// polls (0: 2^22) or when another warp of the group has.
+__device__ __forceinline__ bool pencil_wait(uint64_t* bar, uint32_t parity, int hold,
+                                            volatile int* stop) {
+    if (mbar_try_wait(bar, parity)) return true;
+    for (int i = hold > 0 ? hold : 1 << 22; i > 0; --i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if (*stop) return false;
+    }
+    return false;
+}
+
 // One piece of pass DIR (0 x, 1 y, 2 z) over the job of `a`, by thread group
-// tg of a CTA.  CLO: pieces at CLOSURE ends of the direction are zones.
+// tg of a CTA.  CLO: pieces at CLOSURE ends of the direction are zones.  A wait
+// that gives up sets status bit 2 and *stop; every warp of the group then leaves
+// the piece at its next wait, its own copies in flight waited for, and takes no
+// more.
 template <int DIR, typename V, bool UNI, int MODE, bool CLO>
 __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsigned char* smem,
-                                               int tg, unsigned& phase,
+                                               int tg, unsigned& phase, volatile int* stop,
                                                const PencilPiece& piece) {
     const long grp = piece.grp;
     const int p0 = piece.p0, len = piece.len;
@@ -450,9 +467,16 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         __syncwarp();                  // no lane polls for a phase its own warp has yet to end
         ++phase;
     };
-    auto await_last = [&]() {          // all warps ended the phase before this one
+    auto await_last = [&]() -> bool {  // all warps ended the phase before this one
         const unsigned p = phase - 1;
-        if (!mbar_wait_bounded(bars + (p & 1), (p >> 1) & 1)) report_stage_timeout(a);
+        uint64_t* bar = bars + (p & 1);
+        if (__all_sync(0xffffffffu, pencil_wait(bar, (p >> 1) & 1, a.hold_polls, stop))) return true;
+        if (lane == 0) {
+            *stop = 1;
+            report_stage_timeout(a);
+        }
+        cp_async_wait<0>();
+        return false;
     };
     auto run = [&](auto mi) {
         constexpr bool MI = decltype(mi)::value;
@@ -470,7 +494,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         for (int k = 0; k < nch; ++k) {
 #pragma unroll
             for (int i = 0; i < C; ++i) step(mi, base + i);
-            await_last();
+            if (!await_last()) return;
             if (!MI) {
                 const int s = base + 2 * C;
                 split_fetched(k + 2, s < P::SLOTS ? s : s - P::SLOTS);
@@ -483,10 +507,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
             bprev = base;
             base = base + C < P::SLOTS ? base + C : 0;
         }
-        if (MI) {
-            await_last();
-            write_cells(nch - 1, bprev);
-        }
+        if (MI && await_last()) write_cells(nch - 1, bprev);
     };
 
     // ---- prologue: the table of lines, points ms-4 .. ms+3 into the last 8
@@ -671,11 +692,13 @@ __global__ void __launch_bounds__(640, 1)
     pencil_rhs_kernel(const __grid_constant__ RhsArgs a, int krk) {
     extern __shared__ __align__(16) unsigned char pencil_smem[];
     __shared__ PencilShare sh;
+    __shared__ int stop[2];
     constexpr size_t G = PencilLayout<V>::template bytes<MODE>();
     if (threadIdx.x == 0) {
         int L = 0;
         pencil_share(sh, pencil_work<DIR, PencilLayout<V>::GL>(a, L));
-        pencil_init_bars(pencil_smem + G - 16, G);
+        pencil_init_bars(pencil_smem + G - 16, G, a.hold_polls > 0);
+        stop[0] = stop[1] = 0;
     }
     __syncthreads();
     const int tg = threadIdx.x >= 320;
@@ -690,8 +713,9 @@ __global__ void __launch_bounds__(640, 1)
             }, [&](int, int p0, int L) { return pencil_stop<DIR, CLO>(a, p0, L); });
         pencil_sync(tg);                   // the piece is known, the last one is out
         const PencilPiece& p = sh.piece[tg];
-        if (p.len == 0) break;
-        pencil_segment<DIR, V, UNI, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, p);
+        volatile int* gave_up = &stop[tg];
+        if (p.len == 0 || *gave_up) break;
+        pencil_segment<DIR, V, UNI, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, gave_up, p);
     }
 }
 
@@ -700,17 +724,22 @@ __global__ void __launch_bounds__(640, 1)
 // cross grids; each group copies the arguments of its piece's grid (without
 // the tensor maps) to shared memory.
 constexpr int kArgWords = (int)(offsetof(RhsArgs, tma) / 4);
+static_assert(offsetof(RhsArgs, hold_polls) < offsetof(RhsArgs, tma) &&
+              offsetof(RhsArgs, gk) < offsetof(RhsArgs, tma) && offsetof(RhsArgs, tma) % 4 == 0,
+              "the line passes' arguments come before the maps");
 template <int DIR, typename V, int MODE, bool CLO>
 __global__ void __launch_bounds__(640, 1)
     pencil_batch_kernel(const RhsArgs* __restrict__ grids, const long* __restrict__ woff, int n,
                         int krk) {
     extern __shared__ __align__(16) unsigned char pencil_smem[];
     __shared__ PencilShare sh;
+    __shared__ int stop[2];
     __shared__ __align__(64) uint32_t argw[2][(kArgWords + 15) / 16 * 16];
     constexpr size_t G = PencilLayout<V>::template bytes<MODE>();
     if (threadIdx.x == 0) {
         pencil_share(sh, woff[n]);
-        pencil_init_bars(pencil_smem + G - 16, G);
+        pencil_init_bars(pencil_smem + G - 16, G, grids[0].hold_polls > 0);
+        stop[0] = stop[1] = 0;
     }
     __syncthreads();
     const int tg = threadIdx.x >= 320;
@@ -732,7 +761,13 @@ __global__ void __launch_bounds__(640, 1)
             }, [&](int grid, int p0, int L) { return pencil_stop<DIR, CLO>(grids[grid], p0, L); });
         pencil_sync(tg);                   // the piece is known, the last one is out
         const PencilPiece& p = sh.piece[tg];
+        volatile int* gave_up = &stop[tg];
         if (p.len == 0) break;
+        if (*gave_up) {                    // the pieces it would have taken: reported, not done
+            if (lead) report_stage_timeout(grids[p.grid]);
+            pencil_sync(tg);
+            continue;
+        }
         if (held != p.grid) {
             const uint32_t* src = reinterpret_cast<const uint32_t*>(grids + p.grid);
             for (int w = threadIdx.x - tg * 320; w < kArgWords; w += 320)
@@ -740,7 +775,7 @@ __global__ void __launch_bounds__(640, 1)
             held = p.grid;
             pencil_sync(tg);
         }
-        pencil_segment<DIR, V, true, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, p);
+        pencil_segment<DIR, V, true, MODE, CLO>(a, krk, pencil_smem + tg * G, tg, phase, gave_up, p);
     }
 }
 

@@ -79,16 +79,16 @@ struct RhsArgs {
     // y-, y+, z-, z+: 0 the ghost layer itself, 1 the wrapped and 2 the clamped
     // interior point (the values a ghost fill would have put there)
     int gk[6];
+    // > 0 only in the failure-path test (environment WS_TEST_STAGE_WAIT): the
+    // first staging wait, or the line passes' waits, poll, this many times, an
+    // mbarrier phase that nothing completes, so the kernel takes its timeout
+    // path (status bit 2, early stop) without any fault
+    int hold_polls;
     // TMA staging (tma != 0): per primitive, a map of its LAP array with the
     // (BX+8) x (BY+8) box of a plane and one with the BX x BY centre box.
     // Set only when every box start is 16-byte aligned (even job start x,
     // even pitches, 16-byte aligned fields); otherwise staging uses cp.async.
     int tma;
-    // > 0 only in the failure-path test (environment WS_TEST_STAGE_WAIT):
-    // the first staging wait polls, this many times, an mbarrier nothing
-    // arrives on, so the kernel takes its timeout path (status bit 2, early
-    // stop) without any fault
-    int hold_polls;
     CUtensorMap tm_box[5], tm_ctr[5];
 };
 
