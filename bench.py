@@ -535,7 +535,7 @@ def bench_batch(a, torch, ws, wl, stream):
         ms = e0.elapsed_time(e1)
         st = b.status()
         b.close()
-        pencil = tile[0] < 0 or tile[2] < 0
+        pencil = tile[0] < 0
         res[name] = {"value": cells * 3 * a.batch_steps / (ms * 1e-3) / 1e9,
                      "unit": "Gcell-RHS/s", "ms_per_step": ms / a.batch_steps,
                      "tile": list(tile),

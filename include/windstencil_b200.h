@@ -129,11 +129,12 @@ typedef struct ws_metrics {
 
 /* Kernel selection.  All zeros (the default) and tile_x < 0 select the line
  * passes: three passes (x, y, z) in which each lane marches one grid line
- * (with tile_x < 0, threads = 0, or 256 in FP64 and 512 mixed).  Any other
+ * (with tile_x < 0, threads must be 0, or 256 in FP64 and 512 mixed, which have
+ * no effect).  Any other
  * tile_x, tile_y, threads select the fused tile sweep: a CTA of `threads`
  * threads owns tile_x x tile_y columns and sweeps them along z; scan_z caps
- * the planes of one sweep (0: no cap, each persistent CTA sweeps its whole
- * share of planes; < 0: the line passes instead).  Both give the same results
+ * the planes of one sweep (<= 0: no cap, each persistent CTA sweeps its whole
+ * share of planes).  Both give the same results
  * to rounding, CLOSURE faces included. */
 typedef struct ws_tile {
     int32_t tile_x, tile_y, scan_z, threads;
@@ -453,9 +454,10 @@ WS_API int  ws_blocks_status(ws_blocks* b, int* status, ws_stream_t stream);
 
 /* ------------------------------------------------------------------------ */
 /* Many independent grids, device-resident, stepped together: per RK stage   */
-/* one batched ghost fill, one persistent fused-RHS launch over all grids,   */
-/* one batched stage update; the step is replayed from a CUDA graph.  No     */
-/* reference counterpart (the reference solves one grid per MPI rank).       */
+/* one launch over all grids of each line pass, the last with the stage      */
+/* update (with a tile shape a batched ghost fill and one fused launch); the */
+/* step is replayed from a CUDA graph.  No reference counterpart (the        */
+/* reference solves one grid per MPI rank).                                  */
 /* All grids: Cartesian (metrics_uniform = 1), one precision, no EXTERNAL   */
 /* faces.                                                                    */
 /* ------------------------------------------------------------------------ */
@@ -482,7 +484,7 @@ WS_API int  ws_batch_step(ws_batch* b, int nsteps, ws_stream_t stream);
 /* per-grid status (0, WS_ERR_NONFINITE or WS_ERR_TIMEOUT); synchronises `stream` */
 WS_API int  ws_batch_status(ws_batch* b, int* status, ws_stream_t stream);
 /* times the line passes and the compiled tile shapes on this batch's RHS and
- * keeps the fastest; *chosen is its tile selection (scan_z = -1: the line
+ * keeps the fastest; *chosen is its tile selection (tile_x = -1: the line
  * passes) */
 WS_API int  ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream);
 

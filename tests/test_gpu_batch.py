@@ -74,10 +74,16 @@ def test_batch_autotune_keeps_results(cuda):
     b.rhs()
     before = [b.get_rhs(i) for i in range(len(grids))]
     tile = b.autotune()
-    assert (tile[0], tile[1], tile[3]) in {(16, 8, 768), (16, 8, 704), (8, 8, 256), (8, 8, 384)}
+    lines = tile == (-1, 0, 0, 0)
+    assert lines or (tile[0], tile[1], tile[3]) in {(16, 8, 768), (16, 8, 704), (8, 8, 256),
+                                                    (8, 8, 384)}
     b.rhs()
     for i in range(len(grids)):
-        assert np.array_equal(b.get_rhs(i), before[i])
+        # the batch starts on the line passes; the two kernels agree to rounding
+        if lines:
+            assert np.array_equal(b.get_rhs(i), before[i])
+        else:
+            assert rel_linf(b.get_rhs(i), before[i]).max() <= 1e-12
     b.close()
 
 

@@ -251,18 +251,14 @@ int tile_index(const ws_grid* g, ws_tile tile, bool stage, int* cfg) {
 // Fill RhsArgs and launch; shared by the drop-in entry and the solver.
 bool use_pencil(const ws_grid* g, ws_tile tile) {
     (void)g;
-    if (tile.tile_x < 0 || tile.scan_z < 0) return true;
+    if (tile.tile_x < 0) return true;
     return !(tile.tile_x || tile.tile_y || tile.threads);
 }
 
 namespace {
-// tile_x < 0 may name the warps per CTA that a line pass has always run with
-// (8 in FP64, 16 mixed) or leave them open
+// threads of a selection by tile_x < 0: 0, or the 8 (FP64) or 16 (mixed) warps
+// that the line passes' first form ran with, which are taken and have no effect
 int check_pencil(const ws_grid* g, ws_tile tile) {
-    if (tile.tile_x >= 0) {
-        int cfg = 0;
-        return tile_index(g, tile, false, &cfg);
-    }
     if (tile.threads % 32) return fail(WS_ERR_INVALID, "line passes: threads = 32 x warps");
     const int warps = g->precision == WS_MIXED ? 16 : 8;
     if (tile.threads > 0 && tile.threads / 32 != warps)

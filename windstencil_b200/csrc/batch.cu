@@ -181,7 +181,7 @@ int batch_kernel_cfg(const std::vector<GridState*>& grids, ws_tile tile) {
     if (tile.tile_x < 0) return -1;
     if (tile.tile_x || tile.tile_y || tile.threads) {
         const int c = find_tile_cfg(tile.tile_x, tile.tile_y, tile.threads);
-        return c < 0 ? -2 : tile.scan_z < 0 ? -1 : c;
+        return c < 0 ? -2 : c;
     }
     return -1;
 }
@@ -574,12 +574,11 @@ int ws_batch_status(ws_batch* b, int* status, ws_stream_t stream) {
     return WS_OK;
 }
 
-// Times the candidate kernels on the first RK stage of this batch (ghost
-// fill + RHS and stage update; the current state is left as it was) and
-// keeps the fastest; returns its tile selection in *chosen.  Candidates: the
-// line passes (the default tile shape with scan_z = -1, which any set_tile
-// takes as the line passes) and every compiled tile shape of the fused kernel
-// with two sweep caps.
+// Times the candidate kernels on the first RK stage of this batch (the RHS and
+// stage update, with the tile sweep's ghost fill; the current state is left as
+// it was) and keeps the fastest; returns its tile selection in *chosen.
+// Candidates: the line passes (tile_x = -1) and every compiled tile shape of
+// the fused kernel with two sweep caps.
 int ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream) {
     if (!b) return fail(WS_ERR_INVALID, "batch is NULL");
     cudaStream_t st = (cudaStream_t)stream;
@@ -588,8 +587,7 @@ int ws_batch_autotune(ws_batch* b, ws_tile* chosen, ws_stream_t stream) {
     WS_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     ws_tile best_tile{0, 0, 0, 0};
-    const TileCfg dc = tile_cfg(default_cfg(b->states[0].g.precision, true));
-    std::vector<ws_tile> cand{ws_tile{dc.bx, dc.by, -1, dc.threads}};
+    std::vector<ws_tile> cand{ws_tile{-1, 0, 0, 0}};
     for (int c = 0; c < num_tile_cfgs(); ++c)
         for (int cap : {0, 32}) {
             const TileCfg tc = tile_cfg(c);

@@ -156,7 +156,7 @@ int launch_rhs_pencil_batch(const RhsArgs* g, const long* woff, int n, int preci
 constexpr int kWorkTables = 4;
 long pencil_pass_work(const ws_grid& g, int dir);
 // Whether a launch with tile selection `tile` runs the line passes: an
-// explicit request (tile_x < 0, or a tile shape with scan_z < 0), or the
+// explicit request (tile_x < 0), or the
 // default (all zeros); an explicit fused tile runs the fused kernel.
 bool use_pencil(const ws_grid* g, ws_tile tile);
 
