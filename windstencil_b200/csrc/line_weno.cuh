@@ -27,13 +27,13 @@
 //   so the face value is the central candidate plus
 //     [F_1 (w_0 + w_1) - 3 F_0 w_0 + F_2 (w_3 + w_4) - 3 F_3 w_4] / (12 sum w),
 //   6 operations, and w_0 + w_1, w_3 + w_4 are needed for the sum anyway.
-// * The central candidates of P and M use the same four points, so their sum
-//   is the central formula on the unsplit flux F+ + F-, and the cell's
-//   difference of it is (7 (g_-1 + g_0) - (g_-2 + g_1)) / 12 on the unsplit
-//   flux differences g: 5 operations for both signs.
-// Per face and variable 112 FP64 operations instead of 190.  All of it is an
-// exact algebraic rewrite; in floating point it agrees with the reference's
-// form to a few 1e-16 of the flux.
+// * The central candidates of neighbouring faces difference to
+//   (7 (g_-1 + g_0) - (g_-2 + g_1)) / 12 on the split flux's first differences g:
+//   with the sum of the corrections' difference 5 operations per cell and sign.
+// Per face, variable and sign 51 FP64 operations, 4 for the quotient and 5 for
+// the cell: 120 for both signs instead of 190.  All of it is an exact algebraic
+// rewrite; in floating point it agrees with the reference's form to a few 1e-16
+// of the flux.
 //
 // The split: with E_k+- = e_k +- sqrt(e_k^2 + eps^2) (twice the split
 // eigenvalue) every component is a combination of sigma = c1 E1 + E2 + E3,
@@ -52,11 +52,17 @@ template <>
 struct LineVal<double> {
     using CT = double;
     static constexpr int NL = 1;      // lines per lane
+    static constexpr double SCALE = 1.0;
 };
 template <>
 struct LineVal<float2> {
     using CT = float;
     static constexpr int NL = 2;
+    // the split fluxes are scaled by this power of two (and eps' by its square),
+    // so that products of two indicators stay in the FP32 range up to flux
+    // differences of 5e9; the face-by-face form's pairs did up to 6e8 or 1e9,
+    // these pairs without it, one of them with the largest indicator, 3e8
+    static constexpr double SCALE = 0.0625;
 };
 
 // (the _rn forms are never contracted, so every kernel instance rounds alike)
@@ -115,7 +121,8 @@ __device__ __forceinline__ V lkc() {
     if constexpr (sizeof(typename LineVal<V>::CT) == 8) {
         return lkd[I];
     } else {
-        constexpr float c = (float)lk::val[I];
+        constexpr float c =
+            (float)(lk::val[I] * (I == lk::EPS ? LineVal<V>::SCALE * LineVal<V>::SCALE : 1.0));
         return f2(c);
     }
 }
@@ -261,12 +268,14 @@ __device__ __forceinline__ V weno_push(WenoLine<V>& s, V tn, V& num, V& den) {
 
 // num / den.  FP64: a third-order Newton (Householder) step on the hardware's
 // reciprocal approximation (relative error below 2^-20, so below 2^-60 after
-// the step), 4 operations, within 2 ulp of the quotient, which is a correction
-// to the central value.  No range test: den is a sum of products of four
-// indicators, each at least eps' = 9e-11, so it is never small, and it stays
-// below 2^1022 (where the approximation would underflow) for flux differences
-// up to 1e38; beyond, the products overflow.  A branch here would keep the
-// compiler from overlapping neighbouring points.
+// the step), 4 operations, within 2 ulp of the quotient (one rounding each of the
+// step and the product), which is a correction to the central value.  No range
+// test: den is a sum of products of four indicators, each at least eps' = 9e-11,
+// so it is never small; num, such a product times a flux difference, overflows
+// before den reaches 2^1022, where the approximation would underflow, and does so
+// from flux differences of 1e33 on (alternating signs: 2e33; a single jump: 1e34).
+// The face-by-face form, which shared P's and M's division, overflowed from 1e17
+// on.  A branch here would keep the compiler from overlapping neighbouring points.
 __device__ __forceinline__ double weno_quot(double n, double d) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));

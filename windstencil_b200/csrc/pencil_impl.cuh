@@ -276,7 +276,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         double t0[NL], t0c[NL], kc[NL];
 #pragma unroll
         for (int h = 0; h < NL; ++h) {
-            t0[h] = vmul(e[0][h], 0.5 * a.hrg);
+            t0[h] = vmul(e[0][h], 0.5 * a.hrg * LineVal<V>::SCALE);
             t0c[h] = vmul(t0[h], e[4][h]);
             kc[h] = vmul(t0c[h], vmul(0.5 + a.c3, e[4][h]));
         }
@@ -359,7 +359,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
         }
         if (ADD) cp_async_commit();
     };
-    const double rh = (DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz)) * (FACE ? 1.0 : 1.0 / 12.0);
+    const double rh = (DIR == 0 ? a.rhx : (DIR == 1 ? a.rhy : a.rhz)) * (FACE ? 1.0 / LineVal<V>::SCALE : 1.0 / 12.0);
     // result of this thread's point of chunk k at slot `base`
     auto write_cells = [&](int k, int base) {
         const int i = k * C + sx;
@@ -571,7 +571,9 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
 #pragma unroll 1
             for (int jh = 0; jh < 5 * NL; ++jh) {
                 const int j = jh / NL, h = jh - j * NL;
-                auto t = [&](int i) { return (double)reinterpret_cast<const CT*>(col + i * RS)[h]; };
+                auto t = [&](int i) {
+                    return (double)reinterpret_cast<const CT*>(col + i * RS)[h] / LineVal<V>::SCALE;
+                };
                 double v;
                 if (j == inner) {
                     v = (double)reinterpret_cast<const CT*>(&q)[h];
@@ -586,7 +588,7 @@ __device__ __forceinline__ void pencil_segment(const RhsArgs& a, int krk, unsign
                     } else {
                         v = pencil_closure(t, minus, f0 + j, n, hi);
                     }
-                    if (!FACE) v *= 12.0;
+                    v *= FACE ? LineVal<V>::SCALE : 12.0;
                 }
                 *val(j, h, warp, lane) = v;
             }
