@@ -6,8 +6,8 @@ configuration "Plain FP64 fused RHS at 600x128x128 and 480x512x64": 4 ghost
 cells, periodic in y and z, zero-gradient extrapolation in x, seeded Sod
 state (left rho=1, p=1; right rho=0.125, p=0.1; 1% noise), SSP-RK3 at CFL
 0.5.  One bench step = one SSP-RK3 time step = 3 RHS evaluations, each a
-ghost fill and the x, y and z line passes, the last applying the stage update
-(12 launches), replayed from a CUDA graph.
+the x, y and z line passes, the last applying the stage update (9 launches),
+replayed from a CUDA graph.
 
   value          Gcell-RHS/s = cells x 3 x K / device time of K steps
                  (CUDA events, max over ranks; the state is 1.2 GB > L2, so
@@ -17,8 +17,10 @@ ghost fill and the x, y and z line passes, the last applying the stage update
                  steps, and downloads it again
   roofline       one RHS (the three line passes) through the drop-in entry
                  point, timed with CUDA events on its launch stream;
-                 algorithmic FLOP = 7266 per cell (the oracle's operation
-                 count); FP64-pipe bound, peak = FP64 FMA throughput measured
+                 achieved counts the passes' own FP64 operations, 1974 per
+                 cell, at an FMA's two FLOP each, so that frac is a share of
+                 the FP64 pipe's slots (the oracle's form has 7266 FLOP per
+                 cell); peak = FP64 FMA throughput measured
                  in this run by a DFMA microkernel (MEASURED_PEAKS.json has no
                  FP64 figure); the HBM side uses MEASURED_PEAKS hbm_gbs
   cpu_baseline   the reference's own scalar kernels built for the host
@@ -61,6 +63,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 FLOP_PER_CELL = 7266.0      # oracle or_op_counts(): algorithmic FLOP per cell-RHS
+# operations of the line passes per cell-RHS, each one slot of its pipe: 3 directions x
+# (5 variables x (60 F+ + 59 F-) + 63 for the splits) in FP64; in the mixed form 3 x
+# (5 x (54 + 53) + 59) FP32 ones on packed pairs of lines
+FP64_OPS_PER_CELL = 1974.0
+FP32_OPS_PER_CELL = 1782.0
 BYTES_PER_CELL = 80.0       # 5 FP64 primitives in + 5 FP64 du out (Cartesian metrics)
 
 
@@ -365,13 +372,15 @@ def bench_mixed(a, torch, ws, wl, stream):
         "fp32_peak_tflops_measured": peak32,
         "rhs_gcell_s": cells / (out["mixed_kernel_ms"] * 1e-3) / 1e9})
     # the mixed RHS against the FP32 FMA peak measured now (its reconstruction
-    # runs as packed FP32x2 FMAs; the face difference and stage stay FP64)
-    ach = FLOP_PER_CELL * cells / (out["mixed_kernel_ms"] * 1e-3) / 1e12
+    # runs as packed FP32x2 operations, two FLOP each and line counted; the face
+    # difference and stage stay FP64)
+    ach = 2 * FP32_OPS_PER_CELL * cells / (out["mixed_kernel_ms"] * 1e-3) / 1e12
     res["roofline"] = {"bound": "fp32", "achieved": ach, "peak": peak32, "unit": "TFLOP/s",
                        "frac": ach / peak32 if peak32 else None,
                        "kernel": "line passes x, y, z (mixed form), one RHS",
                        "kernel_ms": out["mixed_kernel_ms"],
                        "peak_source": "FP32 FMA microkernel measured in this run (of measured)",
+                       "fp32_operations_per_cell": FP32_OPS_PER_CELL,
                        "algorithmic_flop_per_cell": FLOP_PER_CELL}
     return res
 
@@ -398,11 +407,12 @@ def bench_second_grid(a, torch, ws, wl, stream, peak64):
         e1.synchronize()
         sms = e0.elapsed_time(e1) / 20
         s.close()
-        tf = FLOP_PER_CELL * cells / (kms * 1e-3) / 1e12
+        tf = 2 * FP64_OPS_PER_CELL * cells / (kms * 1e-3) / 1e12
         res[name] = {"kernel_ms": kms, "rhs_gcell_s": cells / (kms * 1e-3) / 1e9,
                      "step_ms": sms, "value": cells * 3 / (sms * 1e-3) / 1e9,
-                     "unit": "Gcell-RHS/s", "achieved_tflops": tf}
+                     "unit": "Gcell-RHS/s"}
         if name == "fp64":
+            res[name]["achieved_tflops"] = tf
             res[name]["frac_of_fp64_peak"] = tf / peak64 if peak64 else None
     res["kernel_speedup_mixed_vs_fp64"] = res["fp64"]["kernel_ms"] / res["mixed"]["kernel_ms"]
     return res
@@ -541,7 +551,7 @@ def bench_batch(a, torch, ws, wl, stream):
                      "tile": list(tile),
                      "kernel": "line passes (x, y, z)" if pencil else "fused tile sweep",
                      "nonfinite_grids": int(sum(1 for x in st if x)),
-                     "launches_per_step": 12 if pencil else 6}
+                     "launches_per_step": 9 if pencil else 6}
     # one grid at a time, FP64, same grids (a sample of them), same steps:
     # device time of the steps alone, and each request end to end (state
     # upload from host memory, dt, the steps, result download; wall clock)
@@ -744,12 +754,12 @@ def run_ours(a, rank, world, dist):
     f0 = wl.sod_state(a.nx, a.ny, a.nz, seed=2 + rank)
     stream = torch.cuda.Stream()
     if world == 1:
-        # one grid: the step's graphs (ghost fill + x, y, z line passes with the stage, x3)
+        # one grid: the step's graphs (x, y, z line passes with the stage, x3)
         g = ws.Grid(a.nx, a.ny, a.nz, faces=faces)
         s = ws.Solver(g)
         s.set_state(f0, stream=stream)
         dt = s.compute_dt(0.5, stream=stream)
-        launches_per_step = 12      # 3 x (ghost fill + x, y, z line passes)
+        launches_per_step = 9       # 3 x (x, y, z line passes)
 
         def run_steps(n):
             s.step(dt, n, stream=stream)
@@ -800,7 +810,7 @@ def run_ours(a, rank, world, dist):
     # ---- dominant kernel alone (drop-in entry point, same stream)
     rhs_ms = time_rhs_kernel(torch, ws, g, s, stream, max(3, min(a.steps, 20)))
     peak = _peak(ws, "fp64")
-    achieved = FLOP_PER_CELL * cells / (rhs_ms * 1e-3) / 1e12
+    achieved = 2 * FP64_OPS_PER_CELL * cells / (rhs_ms * 1e-3) / 1e12
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -808,10 +818,10 @@ def run_ours(a, rank, world, dist):
         pass
     roof = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak if peak else None, "traffic": measured_traffic(a),
-            "kernel": "one RHS = pencil_x_coop_kernel<8,double,1,0> + "
-                      "pencil_rhs_kernel<1|2,8,double,1,1> (x, y, z line passes)",
+            "kernel": "one RHS = pencil_rhs_kernel<0|1|2,double> (x, y, z line passes)",
             "kernel_ms": rhs_ms,
             "peak_source": "DFMA microkernel measured in this run (of measured)",
+            "fp64_operations_per_cell": FP64_OPS_PER_CELL,
             "algorithmic_flop_per_cell": FLOP_PER_CELL,
             "algorithmic_bytes_per_cell": BYTES_PER_CELL,
             "rhs_gcell_s": cells / (rhs_ms * 1e-3) / 1e9,

@@ -30,8 +30,8 @@
 // * The central candidates of neighbouring faces difference to
 //   (7 (g_-1 + g_0) - (g_-2 + g_1)) / 12 on the split flux's first differences g:
 //   with the sum of the corrections' difference 5 operations per cell and sign.
-// Per face, variable and sign 51 FP64 operations, 4 for the quotient and 5 for
-// the cell: 120 for both signs instead of 190.  All of it is an exact algebraic
+// Per face and variable 51 FP64 operations for F+ and 50 for F-, 4 each for the
+// quotient and 5 for the cell: 119 instead of 190.  All of it is an exact algebraic
 // rewrite; in floating point it agrees with the reference's form to a few 1e-16
 // of the flux.
 //

@@ -27,15 +27,15 @@
 // Why this split: with all five variables in one lane (the earlier form) the
 // reconstruction could keep nothing between faces, so each face took 190 FP64
 // operations from a ring of splits that also held the SM to 8 warps.  One
-// sign of one variable fits 96 registers: 20 warps per SM and 118 operations
+// sign of one variable fits 96 registers: 20 warps per SM and 119 operations
 // per face.  Both signs in a lane would take 112, but their state spilled (10
 // warps at 168 registers: y pass 1.14 ms at 600x128x128, 15 warps at 128: 1.36
-// ms).  Measured at 600x128x128, earlier form -> this one: FP64 x .980 -> .543,
-// y .808 -> .585, z .818 -> .585, z with the stage .948 -> .632 ms; mixed x .487
-// -> .349, y .363 -> .303, z .373 -> .300 ms.  FP64 pipe 65-68% active (ncu);
-// an FMA with three distinct registers takes it 3 cycles instead of 2, and
-// fixed-latency waits and the exchange take the rest.  du goes through HBM
-// between the passes (~320 B/cell).
+// ms).  Measured at 600x128x128, earlier form -> this one: FP64 x .980 -> .505,
+// y .808 -> .543, z .818 -> .541, z with the stage .948 -> .615 ms; mixed x .487
+// -> .348, y .363 -> .305, z .373 -> .304 ms.  FP64 pipe 68-71% active, FP32 FMA
+// pipe of the mixed form 48-52% (ncu); an FMA with three distinct registers takes
+// the FP64 pipe 3 cycles instead of 2, and fixed-latency waits and the exchange
+// take the rest.  du goes through HBM between the passes (~340 B/cell).
 #pragma once
 #include <algorithm>
 #include <type_traits>
