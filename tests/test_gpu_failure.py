@@ -24,7 +24,6 @@ pytestmark = pytest.mark.gpu
 SHAPE = (64, 32, 16)
 HOLD = "64"
 FUSED = (16, 8, 0, 704)        # the fused kernel's tile shape
-LINES = (-1, 0, 0, 0)
 CL, PE = ws.FACE_CLOSURE, ws.FACE_PERIODIC
 
 
